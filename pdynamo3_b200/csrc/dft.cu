@@ -20,6 +20,7 @@
 #include <cctype>
 #include <cmath>
 #include <cstring>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -94,23 +95,70 @@ __device__ __forceinline__ double pasc_ds(double nu) {
     return t4 * t4 * t2;
 }
 
-constexpr double CELL_REL = 1.0e-30;  // cell functions below this fraction of the grid atom's are cut short
+// Cell functions.  A_k(r) = prod_{j != k} s(nu_kj) of atom k at a point; the partition weight of the
+// point's own atom g is A_g / sum_k A_k.  Every factor has magnitude at most one (a factor at |nu| = 1
+// can round to a tiny negative value), so a product's magnitude only falls as factors join it: the
+// product of an atom k != g is cut once it is below CELL_REL times the part of the sum already formed,
+// which changes the sum by less than 256 x 1e-20 of itself.  What makes the cut early is the order: the
+// atom nearest to the point comes first in the sum (its A is close to one), and the factors of each
+// product run over the atoms by their distance from that atom, because a distant atom's small factors
+// are the ones with the atoms near the point.  The centre of the order is taken per warp (the atom
+// nearest to its first point), so that all lanes read the same elements.
+constexpr double CELL_REL = 1.0e-20;
+constexpr int CELL_U = 4;    // factors formed between two tests of the cut: their loads and series overlap
+constexpr int CELL_M = 16;   // distances of the first atoms of the order kept in shared memory
 
-// Unnormalised cell function A_k(r) = prod_{j != k} s(nu_kj) at distances R[j * rs] (atoms k, j).
-// Every factor has magnitude at most one (a factor at |nu| = 1 can round to a tiny negative value),
-// so the product's magnitude only falls; once it is below tiny the rest of the factors are not
-// formed (tiny = 0: the full product).
-__device__ __forceinline__ double cell_factor(int k, int n, const double *R, int rs, const double *rinv, const double *aij,
-                                              double tiny = 0.0) {
-    double prod = 1.0;
-    const double Rk = R[k * rs];
-    for (int j = 0; j < n && !(fabs(prod) < tiny); ++j) {
-        if (j == k) continue;
-        const double mu = (Rk - R[j * rs]) * rinv[k * n + j];
-        const double nu = mu + aij[k * n + j] * (1.0 - mu * mu);
-        prod *= pasc_s(nu);
+__device__ __forceinline__ double point_dist(const double *__restrict__ xyz, int i, double px, double py, double pz) {
+    const double dx = xyz[3 * i] - px, dy = xyz[3 * i + 1] - py, dz = xyz[3 * i + 2] - pz;
+    return sqrt(dx * dx + dy * dy + dz * dz);
+}
+
+// Atom nearest to the point of the warp's first lane.
+__device__ __forceinline__ int nearest_atom(const double *__restrict__ xyz, int natom, double px, double py, double pz) {
+    double best = 1e300;
+    int at = 0;
+    const int lane = threadIdx.x & 31;
+    px = __shfl_sync(0xffffffffu, px, 0);
+    py = __shfl_sync(0xffffffffu, py, 0);
+    pz = __shfl_sync(0xffffffffu, pz, 0);
+    for (int i = lane; i < natom; i += 32) {
+        const double dx = xyz[3 * i] - px, dy = xyz[3 * i + 1] - py, dz = xyz[3 * i + 2] - pz;
+        const double d = dx * dx + dy * dy + dz * dz;
+        if (d < best) { best = d; at = i; }
     }
-    return prod;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double d = __shfl_xor_sync(0xffffffffu, best, o);
+        const int k = __shfl_xor_sync(0xffffffffu, at, o);
+        if (d < best || (d == best && k < at)) { best = d; at = k; }
+    }
+    return at;
+}
+
+// The product over the atoms in the order ord as its smallest factor mn times the product rest of the
+// others, cut once |rest| is below tiny (0: never).  row[j] = {1/R_kj, a_kj}; dist(r, j) is the point's
+// distance from atom j = ord[r].
+template <typename Dist>
+__device__ __forceinline__ void cell_row(int k, double Rk, int n, const int *__restrict__ ord,
+                                         const double2 *__restrict__ row, Dist dist, double tiny, double &mn, double &rest) {
+    mn = 1.0;
+    rest = 1.0;
+    for (int r = 0; r < n; r += CELL_U) {
+        double s[CELL_U];
+#pragma unroll
+        for (int q = 0; q < CELL_U; ++q) {
+            const int rq = min(r + q, n - 1), j = ord[rq];
+            const double2 p = row[j];
+            const double mu = (Rk - dist(rq, j)) * p.x;
+            const double v = pasc_s(mu + p.y * (1.0 - mu * mu));
+            s[q] = (r + q < n && j != k) ? v : 1.0;
+        }
+#pragma unroll
+        for (int q = 0; q < CELL_U; ++q) {
+            if (s[q] < mn) { rest *= mn; mn = s[q]; } else rest *= s[q];
+        }
+        if (fabs(rest) < tiny) break;
+    }
 }
 
 // Basis function (raw Cartesian) value and derivatives up to second order at a point.
@@ -740,15 +788,18 @@ constexpr double WG_DSMAX = 2.0 * APASC;  // max |ds/dmu| = APASC (1-nu^2)^10 |1
 // threads per block of the weight-gradient kernel: 128 (one grid block) while the distance columns
 // fit in shared memory, else 64 (the grid block in two halves)
 inline int wg_threads(int natom) { return natom <= 200 ? 128 : 64; }
-inline size_t wg_smem(int natom) { return (size_t)(6 + wg_threads(natom)) * natom * sizeof(double); }
+inline size_t wg_smem(int natom) {
+    return (size_t)(6 + wg_threads(natom)) * natom * sizeof(double) + (size_t)(wg_threads(natom) / 32) * natom * sizeof(short);
+}
 
 __global__ void __launch_bounds__(128) weight_grad_kernel(const int *__restrict__ bstart, const int *__restrict__ bcount,
                                                           const int *__restrict__ batom, const int *__restrict__ skip,
                                                           const double *__restrict__ pts, const double *__restrict__ pF,
                                                           int natom, const double *__restrict__ xyz,
-                                                          const double *__restrict__ rinv, const double *__restrict__ aij,
+                                                          const double2 *__restrict__ pij, const int *__restrict__ near,
                                                           double *__restrict__ grad) {
-    extern __shared__ double wsh[];  // gradient 3*natom | coordinates 3*natom | distances natom*tpb
+    // gradient 3*natom | coordinates 3*natom | distances natom*tpb | each warp's kept rows natom
+    extern __shared__ double wsh[];
     const int tpb = blockDim.x;
     double *gsh = wsh, *sxyz = wsh + 3 * natom, *sR = wsh + 6 * natom;
     const int b = blockIdx.x, p = threadIdx.x, lane = p & 31;
@@ -756,6 +807,7 @@ __global__ void __launch_bounds__(128) weight_grad_kernel(const int *__restrict_
     __syncthreads();
     const int np = bcount[b];
     const int g = batom[b];
+    short *keep = reinterpret_cast<short *>(sR + (size_t)natom * tpb) + (p >> 5) * natom;
     double *Rp = sR + p;  // this thread's column: Rp[i * tpb] (private, so no block barriers below)
     for (int base = 0; !skip[b] && base < np; base += tpb) {
         if (base + (p & ~31) >= np) break;  // the whole warp is past the end of the block
@@ -767,52 +819,57 @@ __global__ void __launch_bounds__(128) weight_grad_kernel(const int *__restrict_
             const double dx = sxyz[3 * i] - gx, dy = sxyz[3 * i + 1] - gy, dz = sxyz[3 * i + 2] - gz;
             Rp[i * tpb] = sqrt(dx * dx + dy * dy + dz * dz);
         }
-        // pass 1: A_i = smin_i * srest_i, smin_i the smallest factor of the row
-        double smin[256], srest[256];
-        // the grid atom's row first; another row's rest-product (which only falls) is formed down to
-        // 1e-30 A_g: below that the row changes the sum by less than 1e-30 A_g and is dead in pass 2
-        // (rest x |fac| <= 1e-30 A_g x ef w / A_g), and its stored rest-product bounds the true one
-        double sum = 0.0, ag = 0.0, tiny = 0.0;
+        // pass 1: A_i = smin * srest in the warp's order (cell_row); the grid atom's row first and in
+        // full, the others cut at 1e-20 of the sum formed so far (a cut row's stored rest-product
+        // bounds the true one); a row that is cut for every point of the warp is dead in pass 2
+        // (rest x |fac| <= 1e-20 |ef w|) and not kept at all
+        double smin[256], srest[256];  // of the warp's kept rows, in the order of keep[]
+        const int *ord = near + (size_t)nearest_atom(sxyz, natom, gx, gy, gz) * natom;
+        const auto dist = [&](int, int j) { return Rp[j * tpb]; };
+        int nkeep = 0;
+        double sum = 0.0, ag = 0.0;
         for (int ii = -1; ii < natom; ++ii) {
-            const int i = ii < 0 ? g : ii;
+            const int i = ii < 0 ? g : ord[ii];
             if (ii >= 0 && i == g) continue;
-            const double Ri = Rp[i * tpb];
-            const double *ri = rinv + (size_t)i * natom, *ai = aij + (size_t)i * natom;
-            double mn = 1.0, rest = 1.0;
-            for (int j = 0; j < natom && !(fabs(rest) < tiny); ++j) {
-                if (j == i) continue;
-                const double mu = (Ri - Rp[j * tpb]) * ri[j];
-                const double s = pasc_s(mu + ai[j] * (1.0 - mu * mu));
-                if (s < mn) { rest *= mn; mn = s; } else rest *= s;
-            }
-            smin[i] = mn; srest[i] = rest;
+            const double tiny = CELL_REL * sum;
+            double mn, rest;
+            cell_row(i, Rp[i * tpb], natom, ord, pij + (size_t)i * natom, dist, tiny, mn, rest);
             const double A = mn * rest;
             sum += A;
-            if (ii < 0) { ag = A; tiny = CELL_REL * A; }
+            if (ii < 0) ag = A;
+            if (!__any_sync(0xffffffffu, !(fabs(rest) < tiny))) continue;
+            if (lane == 0) keep[nkeep] = (short)i;
+            smin[nkeep] = mn; srest[nkeep] = rest;
+            ++nkeep;
         }
+        __syncwarp();
         const double pg = ag / sum;
         const bool live = active && ef != 0.0 && pg > 0.0;
         if (!__any_sync(0xffffffffu, live)) continue;
         const double ew = live ? ef * w / (pg * sum) : 0.0;
         double ggx = 0.0, ggy = 0.0, ggz = 0.0;
-        for (int i = 0; i < natom; ++i) {
+        for (int ii = 0; ii < nkeep; ++ii) {
+            const int i = keep[ii];
             const double fac = (i == g) ? ew * (1.0 - pg) : -ew * pg;
-            const double mn = smin[i], rest = srest[i];
+            const double mn = smin[ii], rest = srest[ii];
             const bool rowlive = live && rest * WG_DSMAX * fabs(fac) > WG_TINY;
             if (!__any_sync(0xffffffffu, rowlive)) continue;
             const double Ri = Rp[i * tpb], iRi = 1.0 / Ri;
             const double xi = sxyz[3 * i], yi = sxyz[3 * i + 1], zi = sxyz[3 * i + 2];
-            const double *ri = rinv + (size_t)i * natom, *ai = aij + (size_t)i * natom;
+            const double2 *row = pij + (size_t)i * natom;
             double gix = 0.0, giy = 0.0, giz = 0.0;
+            double2 pn = row[0];  // read one atom ahead
             for (int j = 0; j < natom; ++j) {
+                const double2 pr = pn;
+                pn = row[min(j + 1, natom - 1)];
                 if (j == i) continue;
-                double ifac = 0.0, rij = 0.0, mu = 0.0, Rj = 0.0;
+                double ifac = 0.0, mu = 0.0, Rj = 0.0;
+                const double rij = pr.x;
                 bool sig = false;
                 if (rowlive) {
-                    rij = ri[j];
                     Rj = Rp[j * tpb];
                     mu = (Ri - Rj) * rij;
-                    const double aa = ai[j];
+                    const double aa = pr.y;
                     const double nu = mu + aa * (1.0 - mu * mu);
                     const double dsij = -APASC * pasc_ds(nu) * (1.0 - 2.0 * aa * mu);
                     const double dsf = dsij * fac;
@@ -880,7 +937,8 @@ struct GridData {
     int *bstart = nullptr, *bcount = nullptr, *batom = nullptr, *fun = nullptr, *skip = nullptr;
     long long *foff = nullptr, *voff = nullptr;
     double *bval = nullptr;
-    double *rinv = nullptr, *aij = nullptr;
+    double2 *pij = nullptr;         // natom x natom: {1/R_ij, size adjustment a_ij}
+    int *near = nullptr;            // natom x natom: the atoms by distance from each atom, itself first
     long long nfun_total = 0;
     std::vector<long long> h_foff;  // host copies for work accounting
     std::vector<int> h_bcount;
@@ -991,15 +1049,20 @@ extern "C" int pdg_xc_evaluate(const char *name, int n, const double *rho, const
 
 // One candidate per thread: its shell by binary search over the shell offsets, the point from
 // the shell's Lebedev rule and its Becke-style partition weight (DFTGridWeights_Weight,
-// DFTGridWeights.c:220-258: size-adjusted cell functions of all atoms, normalised).
-__global__ void grid_candidates_kernel(long long ncand, int nrs, const long long *__restrict__ rs_off,
-                                       const int *__restrict__ rs_atom, const int *__restrict__ rs_leb,
-                                       const double *__restrict__ rs_r, const double *__restrict__ rs_w,
-                                       const double *__restrict__ leb, const int *__restrict__ leb_off, int natom,
-                                       const double *__restrict__ xyz, const double *__restrict__ rinv,
-                                       const double *__restrict__ aij, double *__restrict__ cand, int *__restrict__ flag) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= ncand) return;
+// DFTGridWeights.c:220-258: size-adjusted cell functions of all atoms, normalised).  Bound by the FP64
+// pipe and the latency of the factors' loads: the distances of all atoms per thread in shared memory
+// and one factor per test (natom^2 of them for most points, since the cut was taken relative to the
+// own atom's A, tiny far from it) took 41.1 ms for 1.35 M candidates of a 96-atom cluster at two CTAs
+// per SM.
+__global__ void __launch_bounds__(128) grid_candidates_kernel(
+    long long ncand, int nrs, const long long *__restrict__ rs_off, const int *__restrict__ rs_atom,
+    const int *__restrict__ rs_leb, const double *__restrict__ rs_r, const double *__restrict__ rs_w,
+    const double *__restrict__ leb, const int *__restrict__ leb_off, int natom, const double *__restrict__ xyz,
+    const double2 *__restrict__ pij, const int *__restrict__ near, double *__restrict__ cand, int *__restrict__ flag) {
+    __shared__ double cR[CELL_M][128];
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const bool valid = t0 < ncand;
+    const long long t = valid ? t0 : ncand - 1;
     int lo = 0, hi = nrs;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -1010,20 +1073,22 @@ __global__ void grid_candidates_kernel(long long ncand, int nrs, const long long
     const double r = rs_r[s];
     const double px = L[0] * r + xyz[3 * g], py = L[1] * r + xyz[3 * g + 1], pz = L[2] * r + xyz[3 * g + 2];
     const double wraw = rs_w[s] * L[3];
-    extern __shared__ double cR[];  // distances, one column per thread ([atom][thread])
-    const int rs = blockDim.x;
-    double *R = cR + threadIdx.x;
-    for (int i = 0; i < natom; ++i) {
-        const double dx = xyz[3 * i] - px, dy = xyz[3 * i + 1] - py, dz = xyz[3 * i + 2] - pz;
-        R[i * rs] = sqrt(dx * dx + dy * dy + dz * dz);
-    }
-    // the grid atom's cell function first; another atom's is only formed down to 1e-30 of it, which
-    // changes the partition sum by less than 1e-28 of the weight's numerator
-    const double pg = cell_factor(g, natom, R, rs, rinv, aij);
+    const int *ord = near + (size_t)nearest_atom(xyz, natom, px, py, pz) * natom;
+    double *R = &cR[0][threadIdx.x];
+    for (int i = 0; i < min(natom, CELL_M); ++i) R[i * 128] = point_dist(xyz, ord[i], px, py, pz);
+    const auto dist = [&](int rk, int j) { return rk < CELL_M ? R[rk * 128] : point_dist(xyz, j, px, py, pz); };
+    double mn, rest;
+    cell_row(g, point_dist(xyz, g, px, py, pz), natom, ord, pij + (size_t)g * natom, dist, 0.0, mn, rest);
+    const double pg = mn * rest;
     double sum = pg;
-    for (int k = 0; k < natom; ++k)
-        if (k != g) sum += cell_factor(k, natom, R, rs, rinv, aij, CELL_REL * pg);
+    for (int rk = 0; rk < natom; ++rk) {
+        const int k = ord[rk];
+        if (k == g) continue;
+        cell_row(k, dist(rk, k), natom, ord, pij + (size_t)k * natom, dist, CELL_REL * sum, mn, rest);
+        sum += mn * rest;
+    }
     const double w = wraw * (pg / sum);
+    if (!valid) return;
     cand[4 * t] = px; cand[4 * t + 1] = py; cand[4 * t + 2] = pz; cand[4 * t + 3] = w;
     flag[t] = fabs(w) > 1.0e-30 ? 1 : 0;
 }
@@ -1268,13 +1333,12 @@ extern "C" int pdg_grid_build(pdg_context *ctx, int accuracy, int n_radial, int 
     }
     aoff[na] = ncand;
     // ---- partition weights on the device ----
-    std::vector<double> rinv((size_t)na * na, 0.0), aij((size_t)na * na, 0.0);
+    std::vector<double2> pij((size_t)na * na, double2{0.0, 0.0});
     for (int i = 0; i < na; ++i)
         for (int j = 0; j < na; ++j) {
             if (i == j) continue;
             const double dx = ctx->xyz[3 * i] - ctx->xyz[3 * j], dy = ctx->xyz[3 * i + 1] - ctx->xyz[3 * j + 1],
                          dz = ctx->xyz[3 * i + 2] - ctx->xyz[3 * j + 2];
-            rinv[i * na + j] = 1.0 / std::sqrt(dx * dx + dy * dy + dz * dz);
             const int zi = ctx->atomic_numbers.empty() ? (int)std::lround(ctx->Z[i]) : ctx->atomic_numbers[i];
             const int zj = ctx->atomic_numbers.empty() ? (int)std::lround(ctx->Z[j]) : ctx->atomic_numbers[j];
             const double chi = bragg(zi) / bragg(zj);
@@ -1282,10 +1346,20 @@ extern "C" int pdg_grid_build(pdg_context *ctx, int accuracy, int n_radial, int 
             double a = temp / (temp * temp - 1.0);
             if (a > 0.5) a = 0.5;
             if (a < -0.5) a = -0.5;
-            aij[i * na + j] = a;
+            pij[(size_t)i * na + j] = double2{1.0 / std::sqrt(dx * dx + dy * dy + dz * dz), a};
         }
-    PDG_CHECK(pupload(ctx, "grid.rinv", &G.rinv, rinv));
-    PDG_CHECK(pupload(ctx, "grid.aij", &G.aij, aij));
+    std::vector<int> near((size_t)na * na);
+    for (int i = 0; i < na; ++i) {
+        const double2 *pi = &pij[(size_t)i * na];
+        auto key = [&](int x) { return x == i ? HUGE_VAL : pi[x].x; };  // 1/R, the atom itself first
+        std::iota(&near[(size_t)i * na], &near[(size_t)i * na] + na, 0);
+        std::sort(&near[(size_t)i * na], &near[(size_t)i * na] + na, [&](int x, int y) {
+            const double kx = key(x), ky = key(y);
+            return kx > ky || (kx == ky && x < y);
+        });
+    }
+    PDG_CHECK(pupload(ctx, "grid.pij", &G.pij, pij));
+    PDG_CHECK(pupload(ctx, "grid.near", &G.near, near));
     const int nrs = (int)rs_off.size();
     long long *d_rs_off = nullptr, *d_aoff = nullptr;
     int *d_rs_atom = nullptr, *d_rs_leb = nullptr, *d_leb_off = nullptr;
@@ -1306,12 +1380,9 @@ extern "C" int pdg_grid_build(pdg_context *ctx, int accuracy, int n_radial, int 
     int *dapos = (int *)pdg_pool(ctx, "grid.apos", (na + 1) * sizeof(int));
     if (!dcand || !dflag || !dpos || !dbsum || !dapos) { pdg_set_error("pdg_grid_build: allocation failed"); return PDG_ERR_ALLOC; }
     if (ncand > 0) {
-        const int ct = wg_threads(na);
-        const size_t csm = (size_t)ct * na * sizeof(double);
-        PDG_CUDA(pdg_allow_max_smem(grid_candidates_kernel));
-        { grid_candidates_kernel<<<(unsigned)((ncand + ct - 1) / ct), ct, csm, ctx->stream>>>(
-            ncand, nrs, d_rs_off, d_rs_atom, d_rs_leb, d_rs_r, d_rs_w, d_leb, d_leb_off, na, ctx->dbasis.atom_xyz, G.rinv,
-            G.aij, dcand, dflag); pdg_count_launch(); }
+        { grid_candidates_kernel<<<(unsigned)((ncand + 127) / 128), 128, 0, ctx->stream>>>(
+            ncand, nrs, d_rs_off, d_rs_atom, d_rs_leb, d_rs_r, d_rs_w, d_leb, d_leb_off, na, ctx->dbasis.atom_xyz, G.pij,
+            G.near, dcand, dflag); pdg_count_launch(); }
         { scan_block_sums_kernel<<<(unsigned)nscan, SCAN_B, 0, ctx->stream>>>(ncand, dflag, dbsum); pdg_count_launch(); }
         { scan_offsets_kernel<<<1, 32, 0, ctx->stream>>>((int)nscan, dbsum); pdg_count_launch(); }
         { scan_final_kernel<<<(unsigned)nscan, SCAN_B, 0, ctx->stream>>>(ncand, dflag, dbsum, dpos); pdg_count_launch(); }
@@ -1503,7 +1574,7 @@ int pdg_dft_grad_device(pdg_context *ctx, double *d_grad) {
     const size_t wsm = wg_smem(ctx->natom);
     PDG_CUDA(pdg_allow_max_smem(weight_grad_kernel));
     { weight_grad_kernel<<<G.nblk, wg_threads(ctx->natom), wsm, ctx->stream>>>(
-        G.bstart, G.bcount, G.batom, G.skip, G.pts, X.pF, ctx->natom, ctx->dbasis.atom_xyz, G.rinv, G.aij, d_grad); pdg_count_launch(); }
+        G.bstart, G.bcount, G.batom, G.skip, G.pts, X.pF, ctx->natom, ctx->dbasis.atom_xyz, G.pij, G.near, d_grad); pdg_count_launch(); }
     PDG_CUDA(cudaGetLastError());
     return PDG_OK;
 }
