@@ -68,6 +68,13 @@ struct PairList {
     int *shA, *shB;   // shell indices (l(A) >= l(B))
     int *poff, *np;   // primitive-pair offset / count
     double *Q;        // Schwarz bound sqrt(max |(ab|ab)|), true normalisation
+    // The primitive records of the pairs as kets, 32 consecutive pairs of a bucket to a group: primitive j
+    // of lane k of a group that starts at slot o is at [(o + j) * 32 + k] with stride 32 between its
+    // 16-byte parts (grec: 4 parts, grec32: 2), so that a warp whose lanes hold the kets of a group reads
+    // whole lines.  goff[group] is o; groups are numbered through the buckets.
+    const double2 *grec;
+    const float4 *grec32;
+    const int *goff;
 };
 
 // Primitive-pair data (all pair classes share one set of arrays).
@@ -97,12 +104,29 @@ __device__ __forceinline__ double load_arg(const double2 *__restrict__ rec, int 
 // is p - a).
 __device__ __forceinline__ double2 load_arg_a(const double2 *__restrict__ rec, int i) { return __ldg(rec + 4 * i + 3); }
 
+// Primitive slot `slot` of the calling lane's ket in the group layout of PairList.
+__device__ __forceinline__ PairRec load_grec(const double2 *__restrict__ g, size_t slot) {
+    const double2 *r = g + slot * 128 + (threadIdx.x & 31);
+    const double2 a = __ldg(r), b = __ldg(r + 32), c = __ldg(r + 64);
+    return PairRec{a.x, a.y, b.x, b.y, c.x, c.y};
+}
+// Its {cut argument, exponent of the pair's first primitive}.
+__device__ __forceinline__ double2 load_grec_arg_a(const double2 *__restrict__ g, size_t slot) {
+    return __ldg(g + slot * 128 + 96 + (threadIdx.x & 31));
+}
+
 // A primitive pair's single-precision record (two 16-byte loads of PrimPairs::rec32).
 struct PairRec32 {
     float p, PAx, PAy, PAz, Kp, hp, arg;
 };
 __device__ __forceinline__ PairRec32 load_rec32(const float4 *__restrict__ rec, int i) {
     const float4 a = __ldg(rec + 2 * i), b = __ldg(rec + 2 * i + 1);
+    return PairRec32{a.x, a.y, a.z, a.w, b.x, b.y, b.z};
+}
+
+__device__ __forceinline__ PairRec32 load_grec32(const float4 *__restrict__ g, size_t slot) {
+    const float4 *r = g + slot * 64 + (threadIdx.x & 31);
+    const float4 a = __ldg(r), b = __ldg(r + 32);
     return PairRec32{a.x, a.y, a.z, a.w, b.x, b.y, b.z};
 }
 
@@ -138,6 +162,11 @@ struct WorkSub {
     long long cta0;          // first CTA of the launch working on this bucket
     int k0;                  // first ket pair of the bucket in the ket class list
     int lanes;               // lanes per quartet (a power of two, <= 32)
+    // the same quartets as (bra pair, group of 32 kets) items, for the warp-per-bra kernels
+    const long long *woffs;  // prefix sums over bra pairs of their ket groups
+    const int *wbra;         // bra pair of every fourth item
+    long long wtotal;        // items
+    int g0;                  // first ket group of the bucket (PairList::goff)
 };
 struct WorkList {
     int nsub;

@@ -25,6 +25,11 @@ struct QuartetBlock {
         int *cbra;          // device: bra pair of quartet min(4k, total-1), k = 0 .. (total-1)/4 + 1
         int k0, nk;         // the bucket's kets: [k0, k0 + nk) of the ket class list
         int bucket;
+        // (bra pair, group of 32 kets) items of the warp-per-bra kernels
+        long long wtotal;
+        long long *woffs;   // device prefix sums over bra pairs (bra.n + 1)
+        int *wbra;          // device: bra pair of item min(4k, wtotal-1)
+        int g0;             // first ket group of the bucket
     } sub[PDG_NBUCKET];
 };
 
@@ -59,6 +64,7 @@ struct pdg_context {
     PairList pairs[PDG_NPAIRCLASS]{};      // device arrays
     std::vector<double> hostQ[PDG_NPAIRCLASS];     // per class, ordered by bucket then Q descending
     std::vector<int> bucket_start[PDG_NPAIRCLASS]; // per class: first pair of each bucket (PDG_NBUCKET + 1)
+    std::vector<int> bucket_group[PDG_NPAIRCLASS]; // per class: first ket group of each bucket
     std::vector<int> hostPoff[PDG_NPAIRCLASS], hostNp[PDG_NPAIRCLASS];  // sorted pair -> primitive pairs
     std::vector<double> hostArg;                                        // primitive-pair exponent arguments
     PrimPairs pp{};
@@ -163,13 +169,30 @@ inline long long pdg_fill_work(WorkList &w, const QuartetBlock &b, const int (&l
         if (k < b.nsub) {
             const auto &s = b.sub[k];
             const int l = lanes[s.bucket];
-            w.sub[k] = WorkSub{s.offs, s.cbra, s.total, cta, s.k0, l};
+            w.sub[k] = WorkSub{s.offs, s.cbra, s.total, cta, s.k0, l, s.woffs, s.wbra, s.wtotal, s.g0};
             cta += (s.total * l + 127) / 128;
         } else {
-            w.sub[k] = WorkSub{nullptr, nullptr, 0, cta, 0, 1};
+            w.sub[k] = WorkSub{nullptr, nullptr, 0, cta, 0, 1, nullptr, nullptr, 0, 0};
         }
     }
     return cta;
+}
+
+// The same for the warp-per-bra kernels: one warp per (bra pair, ket group) item, four to a CTA.
+inline long long pdg_fill_warp_work(WorkList &w, const QuartetBlock &b) {
+    const int one[PDG_NBUCKET] = {1, 1, 1, 1, 1};
+    pdg_fill_work(w, b, one);
+    long long cta = 0;
+    for (int k = 0; k < PDG_NBUCKET; ++k) {
+        w.sub[k].cta0 = cta;
+        cta += (w.sub[k].wtotal + 3) / 4;
+    }
+    return cta;
+}
+inline long long pdg_warp_items(const QuartetBlock &b) {
+    long long n = 0;
+    for (int k = 0; k < b.nsub; ++k) n += b.sub[k].wtotal;
+    return n;
 }
 
 int pdg_ensure_pairs(pdg_context *ctx);

@@ -87,6 +87,21 @@ std::string cname(const char *base, int c) { return std::string(base) + "." + st
 
 }  // namespace
 
+// The primitive records of a class's pairs in the group layout of PairList: one warp per group of 32
+// pairs, one pair per lane (slots past a pair's own primitives are never read).
+__global__ void __launch_bounds__(128) ket_group_kernel(int ng, const int *__restrict__ goff, const int2 *__restrict__ span,
+                                                        PairList pl, PrimPairs pp, double2 *__restrict__ grec,
+                                                        float4 *__restrict__ grec32) {
+    const int g = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (g >= ng || lane >= span[g].y) return;
+    const int k = span[g].x + lane, p0 = pl.poff[k], np = pl.np[k];
+    for (int j = 0; j < np; ++j) {
+        const size_t slot = (size_t)goff[g] + j;
+        for (int f = 0; f < 4; ++f) grec[slot * 128 + 32 * f + lane] = pp.rec[4 * (p0 + j) + f];
+        for (int f = 0; f < 2; ++f) grec32[slot * 64 + 32 * f + lane] = pp.rec32[2 * (p0 + j) + f];
+    }
+}
+
 // Forget the shell-pair data of the last geometry; the device buffers stay in the context's pool.
 void pdg_free_pairs(pdg_context *ctx) {
     for (int c = 0; c < PDG_NPAIRCLASS; ++c) ctx->pairs[c] = PairList{};
@@ -222,6 +237,35 @@ int pdg_ensure_pairs(pdg_context *ctx) {
         bs.assign(PDG_NBUCKET + 1, n);
         for (int k = n - 1; k >= 0; --k) bs[np_bucket(sN[k])] = k;
         for (int k = PDG_NBUCKET - 1; k >= 0; --k) bs[k] = std::min(bs[k], bs[k + 1]);
+        // the pairs as kets in groups of 32 of a bucket, each group as many primitive slots as its
+        // longest pair (PairList::grec)
+        std::vector<int> goff, gfirst;  // first slot; first pair and pair count, by group
+        auto &bg = ctx->bucket_group[c];
+        bg.assign(PDG_NBUCKET, 0);
+        int slots = 0;
+        for (int kb = 0; kb < PDG_NBUCKET; ++kb) {
+            bg[kb] = (int)goff.size();
+            for (int k = bs[kb]; k < bs[kb + 1]; k += 32) {
+                const int e = std::min(k + 32, bs[kb + 1]);
+                goff.push_back(slots);
+                gfirst.push_back(k);
+                gfirst.push_back(e - k);
+                slots += *std::max_element(sN.begin() + k, sN.begin() + e);
+            }
+        }
+        const int ng = (int)goff.size();
+        if (ng & 1) goff.push_back(0);  // the (first, count) pairs behind start on 8 bytes
+        goff.insert(goff.end(), gfirst.begin(), gfirst.end());
+        int *dg = nullptr;
+        PDG_CHECK(upload(ctx, cname("pairs.goff", c), &dg, goff));
+        double2 *grec = (double2 *)pdg_pool(ctx, cname("pairs.grec", c).c_str(), (size_t)slots * 128 * sizeof(double2));
+        float4 *grec32 = (float4 *)pdg_pool(ctx, cname("pairs.grec32", c).c_str(), (size_t)slots * 64 * sizeof(float4));
+        if (!grec || !grec32) { pdg_set_error("device buffer allocation failed (pairs.grec)"); return PDG_ERR_ALLOC; }
+        { ket_group_kernel<<<(ng + 3) / 4, 128, 0, ctx->stream>>>(ng, dg, reinterpret_cast<const int2 *>(dg + ng + (ng & 1)), pl, ctx->pp, grec, grec32); pdg_count_launch(); }
+        PDG_CUDA(cudaGetLastError());
+        pl.grec = grec;
+        pl.grec32 = grec32;
+        pl.goff = dg;
     }
     return PDG_OK;
 }
@@ -271,19 +315,31 @@ int pdg_build_blocks(pdg_context *ctx, double thr) {
             for (int kb = 0; kb < PDG_NBUCKET; ++kb) {
                 const int k0 = ctx->bucket_start[ck][kb], nk = ctx->bucket_start[ck][kb + 1] - k0;
                 if (nk <= 0) continue;
-                std::vector<long long> offs(Qb.size() + 1, 0);
-                for (size_t i = 0; i < Qb.size(); ++i) offs[i + 1] = offs[i] + pdg_ket_count(ctx, cb, ck, (int)i, k0, nk, thr);
-                if (offs.back() == 0) continue;
+                // quartets, and behind them the (bra, group of 32 kets) items, as prefix sums over the bras
+                const size_t nb = Qb.size();
+                std::vector<long long> offs(2 * (nb + 1), 0);
+                long long *woffs = &offs[nb + 1];
+                for (size_t i = 0; i < nb; ++i) {
+                    const long long cnt = pdg_ket_count(ctx, cb, ck, (int)i, k0, nk, thr);
+                    offs[i + 1] = offs[i] + cnt;
+                    woffs[i + 1] = woffs[i] + (cnt + 31) / 32;
+                }
+                if (offs[nb] == 0) continue;
                 auto &sb = qb.sub[qb.nsub++];
-                sb.total = offs.back();
+                sb.total = offs[nb];
+                sb.wtotal = woffs[nb];
                 sb.k0 = k0;
                 sb.nk = nk;
                 sb.bucket = kb;
+                sb.g0 = ctx->bucket_group[ck][kb];
                 PDG_CHECK(upload(ctx, cname("blocks.offs", nbuf), &sb.offs, offs));
-                const long long nmap = (sb.total - 1) / 4 + 2;
-                sb.cbra = (int *)pdg_pool(ctx, cname("blocks.cbra", nbuf).c_str(), nmap * sizeof(int));
+                sb.woffs = sb.offs + nb + 1;
+                const long long nmap = (sb.total - 1) / 4 + 2, wmap = (sb.wtotal - 1) / 4 + 2;
+                sb.cbra = (int *)pdg_pool(ctx, cname("blocks.cbra", nbuf).c_str(), (nmap + wmap) * sizeof(int));
                 if (!sb.cbra) { pdg_set_error("device buffer allocation failed (blocks.cbra)"); return PDG_ERR_ALLOC; }
-                { bra_map_kernel<<<(unsigned)((nmap + 255) / 256), 256, 0, ctx->stream>>>(sb.offs, (int)Qb.size(), sb.total, nmap, sb.cbra); pdg_count_launch(); }
+                sb.wbra = sb.cbra + nmap;
+                { bra_map_kernel<<<(unsigned)((nmap + 255) / 256), 256, 0, ctx->stream>>>(sb.offs, (int)nb, sb.total, nmap, sb.cbra); pdg_count_launch(); }
+                { bra_map_kernel<<<(unsigned)((wmap + 255) / 256), 256, 0, ctx->stream>>>(sb.woffs, (int)nb, sb.wtotal, wmap, sb.wbra); pdg_count_launch(); }
                 PDG_CUDA(cudaGetLastError());
                 qb.total += sb.total;
                 ++nbuf;

@@ -82,6 +82,10 @@ constexpr int kSplitLanesV[kNLanesV][PDG_NBUCKET] = {
 constexpr int kDefaultLanesV[PDG_NPAIRCLASS][PDG_NPAIRCLASS] = {
     {3, 1, 1, 1, 1, 1}, {1, 1, 1, 1, 1, 1}, {1, 1, 1, 1, 1, 1},
     {1, 1, 1, 1, 1, 1}, {0, 1, 1, 1, 1, 1}, {0, 1, 1, 1, 1, 1}};
+// Lists of at least this many (bra, ket group) items take the warp-per-bra form; one lane then walks all
+// primitives of a quartet, so a shorter list leaves the chip waiting for its longest quartets and keeps
+// several lanes per quartet (4 waters: 1.20 ms so, 1.36 ms with the line at 2368 items).
+constexpr long long kWarpItems = 8192;
 constexpr int kOneLane[PDG_NBUCKET] = {1, 1, 1, 1, 1};
 
 }  // namespace
@@ -464,6 +468,168 @@ __global__ void __launch_bounds__(128) eri_jk_kernel(JKArgs args) {
     }
 }
 
+// Sum over the warp; every lane takes part.
+__device__ __forceinline__ double warp_total(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// One warp per (bra pair, group of 32 kets): a lane holds one quartet.  The bra is the same for all
+// lanes, so its records come as broadcast loads and its J elements leave as one atomic per warp; the
+// kets' records come from the group layout in whole lines, once per ket primitive (outer loop) for all
+// bra primitives.  The form with lanes split over the primitives of a quartet reads both records as
+// gathers, repeats the quartet's preamble in every lane and adds J_ab once per lane to one address; the
+// L1 data pipe was 81-92% busy there, here 48-64% with the FP64 pipe at 31-44%.  J+K build of a 42-atom
+// molecule (266 functions, B3LYP) 15.7 -> 13.4 ms, of a 63-atom one in the mixed mode 73.1 -> 59.6 ms.
+template <int LA, int LB, int LC, int LD, bool DOJ, bool DOK, typename T>
+__global__ void __launch_bounds__(128) eri_jk_warp_kernel(JKArgs args) {
+    const WorkSub ws = pick_sub(args.work);
+    const long long w = ((long long)blockIdx.x - ws.cta0) * 4 + (threadIdx.x >> 5);
+    if (w >= ws.wtotal) return;
+    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
+    const int lane = threadIdx.x & 31;
+    const int ib = bra_of(ws.woffs, ws.wbra, w);
+    const int grp = (int)(w - ws.woffs[ib]);
+    const int cnt = (int)(ws.offs[ib + 1] - ws.offs[ib]), slot = grp * 32 + lane;
+    bool act = slot < cnt;
+    const int ik = ws.k0 + min(slot, cnt - 1);
+    const int A = args.bra.shA[ib], B = args.bra.shB[ib], C = args.ket.shA[ik], D = args.ket.shB[ik];
+    const JKScreen scr = jk_screen<DOJ, DOK>(args, ib, ik, A, B, C, D);
+    act = act && scr.any;
+    const unsigned live = __ballot_sync(0xffffffffu, act);
+    if (live == 0) return;
+    if (args.count32 && args.part == 2 && lane == 0) atomicAdd(args.count32, (unsigned long long)__popc(live));
+    T V[NA * NB * NC * ND];
+#pragma unroll
+    for (int i = 0; i < NA * NB * NC * ND; ++i) V[i] = T(0);
+    if (act) {
+        QuartetGeom g;
+        load_xyz(args.bs, A, g.A);
+        load_xyz(args.bs, B, g.B);
+        load_xyz(args.bs, C, g.C);
+        load_xyz(args.bs, D, g.D);
+        const int pb0 = args.bra.poff[ib], pb1 = pb0 + args.bra.np[ib], npk = args.ket.np[ik];
+        const size_t k0 = args.ket.goff[ws.g0 + grp];
+        for (int j = 0; j < npk; ++j) {
+            if constexpr (std::is_same<T, float>::value) {
+                const QuartetGeom32 g32 = geom32(g);
+                const PairRec32 Kp = load_grec32(args.ket.grec32, k0 + j);
+                for (int xb = pb0; xb < pb1; ++xb) {
+                    const PairRec32 Bp = load_rec32(args.pp.rec32, xb);
+                    if (Bp.arg + Kp.arg > (float)PDG_PRIMITIVE_CUT) continue;
+                    eri_prim32<LA, LB, LC, LD>(Bp, Kp, g32, V);
+                }
+            } else {
+                const double argk = load_grec_arg_a(args.ket.grec, k0 + j).x;
+                const PairRec Kp = load_grec(args.ket.grec, k0 + j);
+                for (int xb = pb0; xb < pb1; ++xb) {
+                    if (load_arg(args.pp.rec, xb) + argk > PDG_PRIMITIVE_CUT) continue;
+                    eri_prim<LA, LB, LC, LD, T>(load_rec(args.pp.rec, xb), Kp, g, V);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    const double uf = args.underflow;
+    if (uf > 0.0) {
+#pragma unroll
+        for (int f = 0; f < NA * NB * NC * ND; ++f) {
+            const double nn = comp_norm(LA, f / (NB * NC * ND)) * comp_norm(LB, f / (NC * ND) % NB) *
+                              comp_norm(LC, f / ND % NC) * comp_norm(LD, f % ND);
+            if (fabs((double)V[f] * nn) <= uf) V[f] = T(0);
+        }
+    }
+    double s = 1.0;
+    if (A == B) s *= 0.5;
+    if (C == D) s *= 0.5;
+    if (args.same && ib == ik) s *= 0.5;
+    const int n = args.n;
+    const int oa = args.bs.sh_bf[A], ob = args.bs.sh_bf[B], oc = args.bs.sh_bf[C], od = args.bs.sh_bf[D];
+    const double *__restrict__ Dm = args.D;
+    const bool doj = DOJ && act && scr.j;
+    if (DOJ && __any_sync(0xffffffffu, doj)) {
+        const double s2 = doj ? 2.0 * s : 0.0;
+        double dcd[NC * ND], jcd[NC * ND];
+#pragma unroll
+        for (int i = 0; i < NC * ND; ++i) {
+            dcd[i] = Dm[(oc + i / ND) * n + od + i % ND];
+            jcd[i] = 0.0;
+        }
+#pragma unroll
+        for (int ia = 0; ia < NA; ++ia)
+#pragma unroll
+            for (int jb = 0; jb < NB; ++jb) {
+                const double dab = Dm[(oa + ia) * n + ob + jb];
+                double jab = 0.0;
+#pragma unroll
+                for (int kl = 0; kl < NC * ND; ++kl) {
+                    const double v = V[(ia * NB + jb) * NC * ND + kl];
+                    jab += v * dcd[kl];
+                    jcd[kl] += v * dab;
+                }
+                jab = warp_total(s2 * jab);
+                if (lane == 0) atomicAdd(&args.J[(oa + ia) * n + ob + jb], jab);
+            }
+        if (doj) {
+#pragma unroll
+            for (int i = 0; i < NC * ND; ++i) atomicAdd(&args.J[(oc + i / ND) * n + od + i % ND], s2 * jcd[i]);
+        }
+    }
+    if (DOK && act && scr.k) {
+        // Kt[a][c] += s V Dbd ; Kt[a][d] += s V Dbc
+#pragma unroll
+        for (int ia = 0; ia < NA; ++ia) {
+            double kac[NC], kad[ND];
+#pragma unroll
+            for (int i = 0; i < NC; ++i) kac[i] = 0.0;
+#pragma unroll
+            for (int i = 0; i < ND; ++i) kad[i] = 0.0;
+#pragma unroll
+            for (int jb = 0; jb < NB; ++jb)
+#pragma unroll
+                for (int kc = 0; kc < NC; ++kc) {
+                    const double dbc = Dm[(ob + jb) * n + oc + kc];
+#pragma unroll
+                    for (int ld = 0; ld < ND; ++ld) {
+                        const double v = V[((ia * NB + jb) * NC + kc) * ND + ld];
+                        kac[kc] += v * Dm[(ob + jb) * n + od + ld];
+                        kad[ld] += v * dbc;
+                    }
+                }
+#pragma unroll
+            for (int kc = 0; kc < NC; ++kc) atomicAdd(&args.K[(oa + ia) * n + oc + kc], s * kac[kc]);
+#pragma unroll
+            for (int ld = 0; ld < ND; ++ld) atomicAdd(&args.K[(oa + ia) * n + od + ld], s * kad[ld]);
+        }
+        // Kt[b][c] += s V Dad ; Kt[b][d] += s V Dac
+#pragma unroll
+        for (int jb = 0; jb < NB; ++jb) {
+            double kbc[NC], kbd[ND];
+#pragma unroll
+            for (int i = 0; i < NC; ++i) kbc[i] = 0.0;
+#pragma unroll
+            for (int i = 0; i < ND; ++i) kbd[i] = 0.0;
+#pragma unroll
+            for (int ia = 0; ia < NA; ++ia)
+#pragma unroll
+                for (int kc = 0; kc < NC; ++kc) {
+                    const double dac = Dm[(oa + ia) * n + oc + kc];
+#pragma unroll
+                    for (int ld = 0; ld < ND; ++ld) {
+                        const double v = V[((ia * NB + jb) * NC + kc) * ND + ld];
+                        kbc[kc] += v * Dm[(oa + ia) * n + od + ld];
+                        kbd[ld] += v * dac;
+                    }
+                }
+#pragma unroll
+            for (int kc = 0; kc < NC; ++kc) atomicAdd(&args.K[(ob + jb) * n + oc + kc], s * kbc[kc]);
+#pragma unroll
+            for (int ld = 0; ld < ND; ++ld) atomicAdd(&args.K[(ob + jb) * n + od + ld], s * kbd[ld]);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Cooperative form for the d-shell classes whose component block (up to 6^4 = 1296 values) does
 // not fit one thread's registers: G lanes of a warp share one shell quartet.
@@ -773,6 +939,13 @@ void launch_jk_p(JKArgs a, const QuartetBlock &b, bool doJ, bool doK, cudaStream
         else if (doJ) launch_jk_group<LA, LB, LC, LD, G, true, false, T>(a, b, st);
         else launch_jk_group<LA, LB, LC, LD, G, false, true, T>(a, b, st);
     } else {
+        if (a.variant < 0 && pdg_warp_items(b) >= kWarpItems) {
+            const long long blocks = pdg_fill_warp_work(a.work, b);
+            if (doJ && doK) { eri_jk_warp_kernel<LA, LB, LC, LD, true, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+            else if (doJ) { eri_jk_warp_kernel<LA, LB, LC, LD, true, false, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+            else { eri_jk_warp_kernel<LA, LB, LC, LD, false, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+            return;
+        }
         constexpr bool SP = jk_split(LA, LB, LC, LD);
         const int v = a.variant >= 0 ? a.variant : pdg_jk_variant[CB][CK].load(std::memory_order_relaxed);
         const long long blocks = pdg_fill_work(a.work, b, SP ? kSplitLanesV[v] : kOneLane);
