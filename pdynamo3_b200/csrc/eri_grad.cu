@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "context.h"
+#include "md.cuh"
 #include "rys.cuh"
 #include "rys2d.cuh"
 
@@ -40,7 +41,7 @@ struct GradArgs {
 // with one array the atomic unit of that slice was 76% busy while the FP64 pipe ran at 8% (the mean
 // over all slices was 1%).  The CTAs therefore add to kGradCopies arrays in turn, spread over the
 // slices, and grad_sum_kernel adds them up.  Gradient of a 42-atom molecule (B3LYP/6-31G*, FP64):
-// 120.0 ms with one array, 41.7 ms with the copies; a 60-atom one in the mixed mode 287 -> 108 ms.
+// 120.0 ms with one array, 41.7 ms with the copies; a 57-atom one in the mixed mode 287 -> 108 ms.
 constexpr int kGradCopies = 128;
 __device__ __forceinline__ double *grad_copy(const GradArgs &a) {
     return a.grad + (size_t)(blockIdx.x & (kGradCopies - 1)) * a.gstride;
@@ -128,42 +129,119 @@ __device__ __forceinline__ void grad_hrr(const R (&G)[LA + LB + 2][LC + LD + 2],
         }
 }
 
-// One shell quartet per P lanes (P = the ket bucket's lane count): the lanes split the primitive
-// quartets and add their nine centre derivatives with shuffles before the first lane adds them to the
-// atom gradients.  T is the arithmetic type of the primitive quartets (float for the quartets of the
-// mixed mode whose Schwarz x |Gamma| bound is below the mixed cut): the centre differences and Gamma
-// are formed in double and rounded once, the Boys argument, Rys rule, recursions, transfers and the
-// accumulation run in T.
-template <int LA, int LB, int LC, int LD, typename T = double>
-__global__ void __launch_bounds__(128) eri_grad_kernel(GradArgs args) {
-    const WorkSub ws = pick_sub(args.work);
-    const int P = ws.lanes;
-    const long long t = ((long long)blockIdx.x - ws.cta0) * blockDim.x / P + (long long)(threadIdx.x / P);
-    const int lane = (int)(threadIdx.x & (P - 1));
-    const int ib = bra_of(ws.offs, ws.cbra, min(t, ws.total - 1));
-    if (t >= ws.total) return;
-    const int ik = ws.k0 + (int)(t - ws.offs[ib]);
+// Classes whose gradient takes Hermite sums instead of the Rys rule: the integrals go one order above the
+// energy's, so up to total angular momentum 3 the Hermite integrals (35) and the quartet's density stay
+// in registers.  The rule of n + 1 nodes there reads 18 to 45 coefficient pairs as gathers per primitive
+// quartet, and each node forms nine derivative products per component.  With the warp-per-bra form below:
+// FP64 gradient of a 42-atom molecule (B3LYP/6-31G*) 41.7 -> 33.7 ms, a 57-atom one in the mixed mode
+// 108 -> 89 ms; the s/p classes run at 46-61% of the FP64 pipe.
+template <int LA, int LB, int LC, int LD>
+__host__ __device__ constexpr bool grad_md() { return LA + LB + LC + LD <= 3; }
+
+// Gamma, its centres and the nine centre derivatives (A, B, C) of one primitive quartet added to g.  T is
+// the arithmetic type (float for the quartets of the mixed mode whose Schwarz x |Gamma| bound is below
+// the mixed cut): the centre differences and Gamma are formed in double and rounded once.  ab = A - B and
+// cd = C - D; ea_ and ec_ are the exponents of the first primitives.
+template <int LA, int LB, int LC, int LD, typename T>
+__device__ __forceinline__ void grad_prim(const PairRec &Rb, double ea_, const PairRec &Rk, double ec_,
+                                          const double (&rA)[3], const double (&rC)[3], const T (&ab)[3],
+                                          const T (&cd)[3], const double (&Gam)[ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)],
+                                          T (&g)[9]) {
+    const T p = T(Rb.p), q = T(Rk.p);
+    T rs;
+    if constexpr (std::is_same<T, float>::value) rs = rsqrtf(p + q);
+    else rs = rsqrt(p + q);
+    const T rppq = rs * rs;
+    const T PQ[3] = {T(Rb.Px - Rk.Px), T(Rb.Py - Rk.Py), T(Rb.Pz - Rk.Pz)};
+    const T pref = T(TWO_PI_POW_2P5) * rs * T(Rb.Kp) * T(Rk.Kp);
+    const T PA[3] = {T(Rb.Px - rA[0]), T(Rb.Py - rA[1]), T(Rb.Pz - rA[2])};
+    const T QC[3] = {T(Rk.Px - rC[0]), T(Rk.Py - rC[1]), T(Rk.Pz - rC[2])};
+    const T r2p = T(Rb.hp), r2q = T(Rk.hp);
+    if constexpr (grad_md<LA, LB, LC, LD>()) {
+        const T PB[3] = {PA[0] + ab[0], PA[1] + ab[1], PA[2] + ab[2]};
+        const T QD[3] = {QC[0] + cd[0], QC[1] + cd[1], QC[2] + cd[2]};
+        T dP[3], da[3], db[3], dc[3], dd[3];
+        const T e = md_gradient<LA, LB, LC, LD, T>(p * q * rppq, PQ, pref, PA, PB, r2p, QC, QD, r2q, Gam, dP, da, db, dc, dd);
+        // P = (a A + b B) / p at fixed A - B; P - A = -(b/p)(A - B), P - B = (a/p)(A - B); exp(-(a b/p) |A-B|^2)
+        const T ap = T(2.0 * ea_ * Rb.hp), bp = T(1) - ap, cq = T(2.0 * ec_ * Rk.hp), dq = T(1) - cq;
+        const T ka = T(-2.0 * ea_) * bp * e, kc = T(-2.0 * ec_) * dq * e;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const T ga = ap * dP[k] + ka * ab[k] - bp * da[k] + ap * db[k];
+            g[k] += ga;
+            g[3 + k] += dP[k] - ga;
+            g[6 + k] += kc * cd[k] - cq * dP[k] - dq * dc[k] + cq * dd[k];
+        }
+        return;
+    }
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     constexpr int LAB = LA + LB + 1, LCD = LC + LD + 1, NR = (LAB + LCD) / 2 + 1;
-    const int A = args.bra.shA[ib], B = args.bra.shB[ib], C = args.ket.shA[ik], D = args.ket.shB[ik];
-    const int atA = args.bs.sh_atom[A], atB = args.bs.sh_atom[B], atC = args.bs.sh_atom[C], atD = args.bs.sh_atom[D];
-    if (atA == atB && atA == atC && atA == atD) return;  // one-centre quartets have no gradient
-    if (grad_skip(args, ib, ik, A, B, C, D)) return;
-    double rA[3], rB[3], rC[3], rD[3];
+    const T ea = T(ea_), eb = T(Rb.p - ea_), ec = T(ec_);
+    const T x = p * q * rppq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+    const T PQx = PQ[0], PQy = PQ[1], PQz = PQ[2], PAx = PA[0], PAy = PA[1], PAz = PA[2];
+    const T ABx = ab[0], ABy = ab[1], ABz = ab[2], CDx = cd[0], CDy = cd[1], CDz = cd[2];
+    T u[NR], w[NR];
+    if constexpr (std::is_same<T, float>::value) rys_roots_f<NR>(x, u, w);
+    else rys_roots<NR>(x, u, w);
+    const T QCx = QC[0], QCy = QC[1], QCz = QC[2];
+    const T a2 = T(2) * ea, b2 = T(2) * eb, c2 = T(2) * ec;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        rA[k] = args.bs.atom_xyz[3 * atA + k]; rB[k] = args.bs.atom_xyz[3 * atB + k];
-        rC[k] = args.bs.atom_xyz[3 * atC + k]; rD[k] = args.bs.atom_xyz[3 * atD + k];
+    for (int r = 0; r < NR; ++r) {
+        const T ur = u[r] * rppq;
+        const T b00 = T(0.5) * ur, b10 = r2p * (T(1) - q * ur), b01 = r2q * (T(1) - p * ur);
+        const T fq = q * ur, fp = p * ur;
+        T Gx[LAB + 1][LCD + 1], Gy[LAB + 1][LCD + 1], Gz[LAB + 1][LCD + 1];
+        rys_vrr<LAB, LCD, T>(Gx, T(1), PAx - fq * PQx, QCx + fp * PQx, b10, b01, b00);
+        rys_vrr<LAB, LCD, T>(Gy, T(1), PAy - fq * PQy, QCy + fp * PQy, b10, b01, b00);
+        rys_vrr<LAB, LCD, T>(Gz, w[r] * pref, PAz - fq * PQz, QCz + fp * PQz, b10, b01, b00);
+        T Ix[LA + 2][LB + 2][LC + 2][LD + 1], Iy[LA + 2][LB + 2][LC + 2][LD + 1], Iz[LA + 2][LB + 2][LC + 2][LD + 1];
+        grad_hrr<LA, LB, LC, LD, T>(Gx, ABx, CDx, Ix);
+        grad_hrr<LA, LB, LC, LD, T>(Gy, ABy, CDy, Iy);
+        grad_hrr<LA, LB, LC, LD, T>(Gz, ABz, CDz, Iz);
+#pragma unroll
+        for (int ia = 0; ia < NA; ++ia)
+#pragma unroll
+            for (int jb = 0; jb < NB; ++jb)
+#pragma unroll
+                for (int kc = 0; kc < NC; ++kc)
+#pragma unroll
+                    for (int ld = 0; ld < ND; ++ld) {
+                        const T gm = T(Gam[((ia * NB + jb) * NC + kc) * ND + ld]);
+                        const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
+                        const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
+                        const int cxx = cart_x(LC, kc), cy = cart_y(LC, kc), cz = cart_z(LC, kc);
+                        const int dx = cart_x(LD, ld), dy = cart_y(LD, ld), dz = cart_z(LD, ld);
+                        const T x0 = Ix[ax][bx][cxx][dx], y0 = Iy[ay][by][cy][dy], z0 = Iz[az][bz][cz][dz];
+                        const T gy = gm * y0 * z0, gx = gm * x0 * z0, gz = gm * x0 * y0;
+                        // centre A
+                        g[0] += gy * (a2 * Ix[ax + 1][bx][cxx][dx] - (ax ? ax * Ix[ax ? ax - 1 : 0][bx][cxx][dx] : T(0)));
+                        g[1] += gx * (a2 * Iy[ay + 1][by][cy][dy] - (ay ? ay * Iy[ay ? ay - 1 : 0][by][cy][dy] : T(0)));
+                        g[2] += gz * (a2 * Iz[az + 1][bz][cz][dz] - (az ? az * Iz[az ? az - 1 : 0][bz][cz][dz] : T(0)));
+                        // centre B
+                        g[3] += gy * (b2 * Ix[ax][bx + 1][cxx][dx] - (bx ? bx * Ix[ax][bx ? bx - 1 : 0][cxx][dx] : T(0)));
+                        g[4] += gx * (b2 * Iy[ay][by + 1][cy][dy] - (by ? by * Iy[ay][by ? by - 1 : 0][cy][dy] : T(0)));
+                        g[5] += gz * (b2 * Iz[az][bz + 1][cz][dz] - (bz ? bz * Iz[az][bz ? bz - 1 : 0][cz][dz] : T(0)));
+                        // centre C
+                        g[6] += gy * (c2 * Ix[ax][bx][cxx + 1][dx] - (cxx ? cxx * Ix[ax][bx][cxx ? cxx - 1 : 0][dx] : T(0)));
+                        g[7] += gx * (c2 * Iy[ay][by][cy + 1][dy] - (cy ? cy * Iy[ay][by][cy ? cy - 1 : 0][dy] : T(0)));
+                        g[8] += gz * (c2 * Iz[az][bz][cz + 1][dz] - (cz ? cz * Iz[az][bz][cz ? cz - 1 : 0][dz] : T(0)));
+                    }
     }
+}
+
+// Gamma = 4 s [D'ab D'cd - (c_x/4)(D'ac D'bd + D'ad D'bc)] of a quartet's component block.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void grad_gamma(const GradArgs &args, int A, int B, int C, int D, bool diag,
+                                           double (&Gam)[ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)]) {
+    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     double s = 1.0;
     if (A == B) s *= 0.5;
     if (C == D) s *= 0.5;
-    if (args.same && ib == ik) s *= 0.5;
+    if (diag) s *= 0.5;
     const int n = args.n;
     const int oa = args.bs.sh_bf[A], ob = args.bs.sh_bf[B], oc = args.bs.sh_bf[C], od = args.bs.sh_bf[D];
     const double *__restrict__ Dm = args.D;
     const double cj = args.doJ ? 4.0 * s : 0.0, ck = -s * args.cx;
-    double Gam[NA * NB * NC * ND];
 #pragma unroll
     for (int ia = 0; ia < NA; ++ia)
 #pragma unroll
@@ -180,8 +258,35 @@ __global__ void __launch_bounds__(128) eri_grad_kernel(GradArgs args) {
                 }
             }
         }
-    const T ABx = T(rA[0] - rB[0]), ABy = T(rA[1] - rB[1]), ABz = T(rA[2] - rB[2]);
-    const T CDx = T(rC[0] - rD[0]), CDy = T(rC[1] - rD[1]), CDz = T(rC[2] - rD[2]);
+}
+
+// One shell quartet per P lanes (P = the ket bucket's lane count): the lanes split the primitive
+// quartets and add their nine centre derivatives with shuffles before the first lane adds them to the
+// atom gradients.  For the lists too short for the warp-per-bra form below.
+template <int LA, int LB, int LC, int LD, typename T = double>
+__global__ void __launch_bounds__(128) eri_grad_kernel(GradArgs args) {
+    const WorkSub ws = pick_sub(args.work);
+    const int P = ws.lanes;
+    const long long t = ((long long)blockIdx.x - ws.cta0) * blockDim.x / P + (long long)(threadIdx.x / P);
+    const int lane = (int)(threadIdx.x & (P - 1));
+    const int ib = bra_of(ws.offs, ws.cbra, min(t, ws.total - 1));
+    if (t >= ws.total) return;
+    const int ik = ws.k0 + (int)(t - ws.offs[ib]);
+    const int A = args.bra.shA[ib], B = args.bra.shB[ib], C = args.ket.shA[ik], D = args.ket.shB[ik];
+    const int atA = args.bs.sh_atom[A], atB = args.bs.sh_atom[B], atC = args.bs.sh_atom[C], atD = args.bs.sh_atom[D];
+    if (atA == atB && atA == atC && atA == atD) return;  // one-centre quartets have no gradient
+    if (grad_skip(args, ib, ik, A, B, C, D)) return;
+    double rA[3], rC[3];
+    T ab[3], cd[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        rA[k] = args.bs.atom_xyz[3 * atA + k];
+        rC[k] = args.bs.atom_xyz[3 * atC + k];
+        ab[k] = T(rA[k] - args.bs.atom_xyz[3 * atB + k]);
+        cd[k] = T(rC[k] - args.bs.atom_xyz[3 * atD + k]);
+    }
+    double Gam[ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)];
+    grad_gamma<LA, LB, LC, LD>(args, A, B, C, D, args.same && ib == ik, Gam);
     T g[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) g[k] = T(0);
@@ -191,71 +296,11 @@ __global__ void __launch_bounds__(128) eri_grad_kernel(GradArgs args) {
     int sb = lane / npk, sk = lane - sb * npk;
     for (int idx = lane; idx < npb * npk; idx += P, sk += P) {
         while (sk >= npk) { sk -= npk; ++sb; }
-        const int jb_ = pb0 + sb, jk = pk0 + sk;
+        const int jb = pb0 + sb, jk = pk0 + sk;
         // the cut arguments and the first exponents of both pairs in two 16-byte loads
-        const double2 xb = load_arg_a(pp.rec, jb_), xk = load_arg_a(pp.rec, jk);
+        const double2 xb = load_arg_a(pp.rec, jb), xk = load_arg_a(pp.rec, jk);
         if (xb.x + xk.x > PDG_PRIMITIVE_CUT) continue;
-        const PairRec Rb = load_rec(pp.rec, jb_), Rk = load_rec(pp.rec, jk);
-        const T ea = T(xb.y), eb = T(Rb.p - xb.y), p = T(Rb.p);
-        const T PAx = T(Rb.Px - rA[0]), PAy = T(Rb.Py - rA[1]), PAz = T(Rb.Pz - rA[2]);
-        {
-            const T ec = T(xk.y), q = T(Rk.p);
-            T rs;
-            if constexpr (std::is_same<T, float>::value) rs = rsqrtf(p + q);
-            else rs = rsqrt(p + q);
-            const T rppq = rs * rs;
-            const T PQx = T(Rb.Px - Rk.Px), PQy = T(Rb.Py - Rk.Py), PQz = T(Rb.Pz - Rk.Pz);
-            const T x = p * q * rppq * (PQx * PQx + PQy * PQy + PQz * PQz);
-            const T pref = T(TWO_PI_POW_2P5) * rs * T(Rb.Kp) * T(Rk.Kp);
-            T u[NR], w[NR];
-            if constexpr (std::is_same<T, float>::value) rys_roots_f<NR>(x, u, w);
-            else rys_roots<NR>(x, u, w);
-            const T QCx = T(Rk.Px - rC[0]), QCy = T(Rk.Py - rC[1]), QCz = T(Rk.Pz - rC[2]);
-            const T r2p = T(Rb.hp), r2q = T(Rk.hp);
-            const T a2 = T(2) * ea, b2 = T(2) * eb, c2 = T(2) * ec;
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const T ur = u[r] * rppq;
-                const T b00 = T(0.5) * ur, b10 = r2p * (T(1) - q * ur), b01 = r2q * (T(1) - p * ur);
-                const T fq = q * ur, fp = p * ur;
-                T Gx[LAB + 1][LCD + 1], Gy[LAB + 1][LCD + 1], Gz[LAB + 1][LCD + 1];
-                rys_vrr<LAB, LCD, T>(Gx, T(1), PAx - fq * PQx, QCx + fp * PQx, b10, b01, b00);
-                rys_vrr<LAB, LCD, T>(Gy, T(1), PAy - fq * PQy, QCy + fp * PQy, b10, b01, b00);
-                rys_vrr<LAB, LCD, T>(Gz, w[r] * pref, PAz - fq * PQz, QCz + fp * PQz, b10, b01, b00);
-                T Ix[LA + 2][LB + 2][LC + 2][LD + 1], Iy[LA + 2][LB + 2][LC + 2][LD + 1], Iz[LA + 2][LB + 2][LC + 2][LD + 1];
-                grad_hrr<LA, LB, LC, LD, T>(Gx, ABx, CDx, Ix);
-                grad_hrr<LA, LB, LC, LD, T>(Gy, ABy, CDy, Iy);
-                grad_hrr<LA, LB, LC, LD, T>(Gz, ABz, CDz, Iz);
-#pragma unroll
-                for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-                    for (int jb = 0; jb < NB; ++jb)
-#pragma unroll
-                        for (int kc = 0; kc < NC; ++kc)
-#pragma unroll
-                            for (int ld = 0; ld < ND; ++ld) {
-                                const T gm = T(Gam[((ia * NB + jb) * NC + kc) * ND + ld]);
-                                const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
-                                const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                                const int cxx = cart_x(LC, kc), cy = cart_y(LC, kc), cz = cart_z(LC, kc);
-                                const int dx = cart_x(LD, ld), dy = cart_y(LD, ld), dz = cart_z(LD, ld);
-                                const T x0 = Ix[ax][bx][cxx][dx], y0 = Iy[ay][by][cy][dy], z0 = Iz[az][bz][cz][dz];
-                                const T gy = gm * y0 * z0, gx = gm * x0 * z0, gz = gm * x0 * y0;
-                                // centre A
-                                g[0] += gy * (a2 * Ix[ax + 1][bx][cxx][dx] - (ax ? ax * Ix[ax ? ax - 1 : 0][bx][cxx][dx] : T(0)));
-                                g[1] += gx * (a2 * Iy[ay + 1][by][cy][dy] - (ay ? ay * Iy[ay ? ay - 1 : 0][by][cy][dy] : T(0)));
-                                g[2] += gz * (a2 * Iz[az + 1][bz][cz][dz] - (az ? az * Iz[az ? az - 1 : 0][bz][cz][dz] : T(0)));
-                                // centre B
-                                g[3] += gy * (b2 * Ix[ax][bx + 1][cxx][dx] - (bx ? bx * Ix[ax][bx ? bx - 1 : 0][cxx][dx] : T(0)));
-                                g[4] += gx * (b2 * Iy[ay][by + 1][cy][dy] - (by ? by * Iy[ay][by ? by - 1 : 0][cy][dy] : T(0)));
-                                g[5] += gz * (b2 * Iz[az][bz + 1][cz][dz] - (bz ? bz * Iz[az][bz ? bz - 1 : 0][cz][dz] : T(0)));
-                                // centre C
-                                g[6] += gy * (c2 * Ix[ax][bx][cxx + 1][dx] - (cxx ? cxx * Ix[ax][bx][cxx ? cxx - 1 : 0][dx] : T(0)));
-                                g[7] += gx * (c2 * Iy[ay][by][cy + 1][dy] - (cy ? cy * Iy[ay][by][cy ? cy - 1 : 0][dy] : T(0)));
-                                g[8] += gz * (c2 * Iz[az][bz][cz + 1][dz] - (cz ? cz * Iz[az][bz][cz ? cz - 1 : 0][dz] : T(0)));
-                            }
-            }
-        }
+        grad_prim<LA, LB, LC, LD, T>(load_rec(pp.rec, jb), xb.y, load_rec(pp.rec, jk), xk.y, rA, rC, ab, cd, Gam, g);
     }
     double gd[9];
 #pragma unroll
@@ -275,6 +320,76 @@ __global__ void __launch_bounds__(128) eri_grad_kernel(GradArgs args) {
         atomicAdd(&gr[3 * atB + k], gd[3 + k]);
         atomicAdd(&gr[3 * atC + k], gd[6 + k]);
         atomicAdd(&gr[3 * atD + k], -(gd[k] + gd[3 + k] + gd[6 + k]));
+    }
+}
+
+// One warp per (bra pair, group of 32 kets), one quartet per lane (see eri_jk_warp_kernel): the bra's
+// records are broadcast loads, the kets' come in whole lines from the group layout, and the derivatives
+// of A and B are summed over the warp before they leave.
+template <int LA, int LB, int LC, int LD, typename T>
+__global__ void __launch_bounds__(128) eri_grad_warp_kernel(GradArgs args) {
+    const WorkSub ws = pick_sub(args.work);
+    const long long w = ((long long)blockIdx.x - ws.cta0) * 4 + (threadIdx.x >> 5);
+    if (w >= ws.wtotal) return;
+    const int lane = threadIdx.x & 31;
+    const int ib = bra_of(ws.woffs, ws.wbra, w);
+    const int grp = (int)(w - ws.woffs[ib]);
+    const int cnt = (int)(ws.offs[ib + 1] - ws.offs[ib]), slot = grp * 32 + lane;
+    const int ik = ws.k0 + min(slot, cnt - 1);
+    const int A = args.bra.shA[ib], B = args.bra.shB[ib], C = args.ket.shA[ik], D = args.ket.shB[ik];
+    const int atA = args.bs.sh_atom[A], atB = args.bs.sh_atom[B], atC = args.bs.sh_atom[C], atD = args.bs.sh_atom[D];
+    const bool act = slot < cnt && !(atA == atB && atA == atC && atA == atD) && !grad_skip(args, ib, ik, A, B, C, D);
+    if (!__any_sync(0xffffffffu, act)) return;
+    T g[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) g[k] = T(0);
+    if (act) {
+        double rA[3], rC[3];
+        T ab[3], cd[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            rA[k] = args.bs.atom_xyz[3 * atA + k];
+            rC[k] = args.bs.atom_xyz[3 * atC + k];
+            ab[k] = T(rA[k] - args.bs.atom_xyz[3 * atB + k]);
+            cd[k] = T(rC[k] - args.bs.atom_xyz[3 * atD + k]);
+        }
+        double Gam[ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)];
+        grad_gamma<LA, LB, LC, LD>(args, A, B, C, D, args.same && ib == ik, Gam);
+        const double2 *__restrict__ rec = args.pp.rec;
+        const int pb0 = args.bra.poff[ib], pb1 = pb0 + args.bra.np[ib], npk = args.ket.np[ik];
+        const size_t k0 = args.ket.goff[ws.g0 + grp];
+        for (int j = 0; j < npk; ++j) {
+            const double2 xk = load_grec_arg_a(args.ket.grec, k0 + j);
+            const PairRec Rk = load_grec(args.ket.grec, k0 + j);
+            for (int jb = pb0; jb < pb1; ++jb) {
+                const double2 xb = load_arg_a(rec, jb);
+                if (xb.x + xk.x > PDG_PRIMITIVE_CUT) continue;
+                grad_prim<LA, LB, LC, LD, T>(load_rec(rec, jb), xb.y, Rk, xk.y, rA, rC, ab, cd, Gam, g);
+            }
+        }
+    }
+    __syncwarp();
+    double *gr = grad_copy(args);
+    double sum[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        sum[k] = (double)g[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    }
+    if (act) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            atomicAdd(&gr[3 * atC + k], (double)g[6 + k]);
+            atomicAdd(&gr[3 * atD + k], -((double)g[k] + (double)g[3 + k] + (double)g[6 + k]));
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            atomicAdd(&gr[3 * atA + k], sum[k]);
+            atomicAdd(&gr[3 * atB + k], sum[3 + k]);
+        }
     }
 }
 
@@ -541,6 +656,10 @@ constexpr int PLB[PDG_NPAIRCLASS] = {0, 0, 1, 0, 1, 2};
 // Lanes per quartet of the one-thread gradient form by ket bucket: the buckets with many primitive
 // pairs split their primitive quartets.
 constexpr int kGradLanes[PDG_NBUCKET] = {1, 1, 2, 4, 4};
+// Lists of at least this many (bra, ket group) items take the warp-per-bra form: every SM then has its
+// resident warps (8 to 16 at these register counts) more than once over; below it one lane per quartet
+// would leave SMs idle.
+constexpr long long kGradWarpItems = 4096;
 
 template <int CB, int CK>
 void launch_grad_t(const GradArgs &a0, const QuartetBlock &b, cudaStream_t st) {
@@ -557,13 +676,21 @@ void launch_grad_t(const GradArgs &a0, const QuartetBlock &b, cudaStream_t st) {
         a.part = 0;  // the cooperative d-class form evaluates every quartet in FP64
         { kern<<<(unsigned)blocks, 128, smem, st>>>(a); pdg_count_launch(); }
     } else {
+        const bool mixed = a.part != 0;
+        if (pdg_warp_items(b) >= kGradWarpItems) {
+            const long long blocks = pdg_fill_warp_work(a.work, b);
+            if (mixed) a.part = 1;
+            { eri_grad_warp_kernel<LA, LB, LC, LD, double><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+            if (!mixed) return;
+            a.part = 2;
+            { eri_grad_warp_kernel<LA, LB, LC, LD, float><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+            return;
+        }
         const long long blocks = pdg_fill_work(a.work, b, kGradLanes);
-        if (a.part == 0) {
-            { eri_grad_kernel<LA, LB, LC, LD, double><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
-        } else {
-            // mixed mode: the quartets above the mixed cut in FP64, the rest in FP32
-            a.part = 1;
-            { eri_grad_kernel<LA, LB, LC, LD, double><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+        // mixed mode: the quartets above the mixed cut in FP64, the rest in FP32
+        if (mixed) a.part = 1;
+        { eri_grad_kernel<LA, LB, LC, LD, double><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+        if (mixed) {
             a.part = 2;
             { eri_grad_kernel<LA, LB, LC, LD, float><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
         }
