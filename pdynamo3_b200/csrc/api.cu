@@ -205,6 +205,10 @@ extern "C" int pdg_context_destroy(pdg_context *ctx) {
     clear_pool(ctx);
     if (ctx->cublas) cublasDestroy(ctx->cublas);
     if (ctx->cusolver) cusolverDnDestroy(ctx->cusolver);
+    for (cudaEvent_t e : ctx->side_event)
+        if (e) cudaEventDestroy(e);
+    for (cudaStream_t s : ctx->side)
+        if (s) cudaStreamDestroy(s);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return PDG_OK;

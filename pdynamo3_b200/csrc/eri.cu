@@ -312,17 +312,21 @@ int pdg_build_blocks(pdg_context *ctx, double thr) {
             QuartetBlock qb{};
             qb.cb = cb;
             qb.ck = ck;
+            const int lt = PLA[cb] + PLB[cb] + PLA[ck] + PLB[ck];
+            const double per = 20.0 + (lt / 2 + 1) * ncart(PLA[cb]) * ncart(PLB[cb]) * ncart(PLA[ck]) * ncart(PLB[ck]);
             for (int kb = 0; kb < PDG_NBUCKET; ++kb) {
                 const int k0 = ctx->bucket_start[ck][kb], nk = ctx->bucket_start[ck][kb + 1] - k0;
                 if (nk <= 0) continue;
                 // quartets, and behind them the (bra, group of 32 kets) items, as prefix sums over the bras
                 const size_t nb = Qb.size();
                 std::vector<long long> offs(2 * (nb + 1), 0);
+                const double npk = ctx->hostNp[ck][k0];
                 long long *woffs = &offs[nb + 1];
                 for (size_t i = 0; i < nb; ++i) {
                     const long long cnt = pdg_ket_count(ctx, cb, ck, (int)i, k0, nk, thr);
                     offs[i + 1] = offs[i] + cnt;
                     woffs[i + 1] = woffs[i] + (cnt + 31) / 32;
+                    qb.cost += per * npk * ctx->hostNp[cb][i] * cnt;
                 }
                 if (offs[nb] == 0) continue;
                 auto &sb = qb.sub[qb.nsub++];
@@ -347,6 +351,8 @@ int pdg_build_blocks(pdg_context *ctx, double thr) {
             if (qb.nsub > 0) ctx->blocks.push_back(qb);
         }
     }
+    // the launches overlap (ClassFork): the longest go first
+    std::stable_sort(ctx->blocks.begin(), ctx->blocks.end(), [](const QuartetBlock &x, const QuartetBlock &y) { return x.cost > y.cost; });
     ctx->blocks_thr = thr;
     return PDG_OK;
 }
@@ -396,6 +402,7 @@ int pdg_eri_jk_screened(pdg_context *ctx, const double *d_D, double *d_J, double
     }
     long long nq = 0;
     ProfScope prof(ctx, "eri_jk");
+    ClassFork fork(ctx);
     for (const auto &b : ctx->blocks) {
         JKArgs a;
         a.bra = ctx->pairs[b.cb];
@@ -417,13 +424,13 @@ int pdg_eri_jk_screened(pdg_context *ctx, const double *d_D, double *d_J, double
         if (mixed) {
             // quartets whose bound Q_AB Q_CD max|D| is below mixed_cut in FP32, the rest in FP64
             a.part = 1;
-            jk_of(b.cb, b.ck)(a, b, doJ, doK, false, ctx->stream);
+            jk_of(b.cb, b.ck)(a, b, doJ, doK, false, fork.stream(b.cost));
             PDG_CUDA(cudaGetLastError());
             a.part = 2;
-            jk_of(b.cb, b.ck)(a, b, doJ, doK, true, ctx->stream);
+            jk_of(b.cb, b.ck)(a, b, doJ, doK, true, fork.stream(b.cost));
         } else {
             a.part = 0;
-            jk_of(b.cb, b.ck)(a, b, doJ, doK, false, ctx->stream);
+            jk_of(b.cb, b.ck)(a, b, doJ, doK, false, fork.stream(b.cost));
         }
         PDG_CUDA(cudaGetLastError());
         nq += b.total;

@@ -6,6 +6,7 @@
 // (GaussianBases/__extensions__/csource/GaussianBasisContainerIntegrals_f2Xf2.c:146-209,337-421)
 // and GaussianBasisIntegrals_f2Cf2r1 (GaussianBasisIntegrals_f2Xf2.c:905-1364), whose density
 // factor 4 s D D - s c_x (D D + D D) is the same Gamma.
+#include <memory>
 #include <type_traits>
 
 #include "context.h"
@@ -729,6 +730,7 @@ int pdg_eri_grad(pdg_context *ctx, const double *d_D, double cx, bool doJ, doubl
     double *part = (double *)pdg_pool(ctx, "grad_part", (size_t)kGradCopies * gstride * sizeof(double));
     if (!part) { pdg_set_error("pdg_eri_grad: device buffer allocation failed"); return PDG_ERR_ALLOC; }
     PDG_CUDA(cudaMemsetAsync(part, 0, (size_t)kGradCopies * gstride * sizeof(double), ctx->stream));
+    auto fork = std::make_unique<ClassFork>(ctx);
     for (const auto &b : ctx->blocks) {
         GradArgs a;
         a.bra = ctx->pairs[b.cb];
@@ -747,9 +749,10 @@ int pdg_eri_grad(pdg_context *ctx, const double *d_D, double cx, bool doJ, doubl
         a.gcut = gcut;
         a.part = ctx->precision_mode == 1 ? 1 : 0;
         a.mixed_cut = ctx->mixed_cut;
-        grad_table[b.cb][b.ck](a, b, ctx->stream);
+        grad_table[b.cb][b.ck](a, b, fork->stream(b.cost));
         PDG_CUDA(cudaGetLastError());
     }
+    fork.reset();
     { grad_sum_kernel<<<(n3 + 31) / 32, 256, 0, ctx->stream>>>(n3, gstride, part, d_grad); pdg_count_launch(); }
     PDG_CUDA(cudaGetLastError());
     return PDG_OK;
