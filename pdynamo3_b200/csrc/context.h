@@ -211,6 +211,20 @@ struct ClassFork {
     ClassFork &operator=(const ClassFork &) = delete;
 };
 
+// Partial gradient arrays.  A molecule has only 3 natom gradient elements (about 1 KB at 42 atoms),
+// which the address hash puts in one or two L2 slices, and every quartet adds twelve values to them:
+// with one array the atomic unit of that slice was 76% busy while the FP64 pipe ran at 8% (the mean
+// over all slices was 1%).  The CTAs therefore add to kGradCopies arrays in turn, spread over the
+// slices, and grad_sum_kernel adds them up.  Gradient of a 42-atom molecule (B3LYP/6-31G*, FP64):
+// 120.0 ms with one array, 41.7 ms with the copies; a 57-atom one in the mixed mode 287 -> 108 ms.
+constexpr int kGradCopies = 128;
+__device__ __forceinline__ double *pdg_grad_copy(double *part, int gstride) {
+    return part + (size_t)(blockIdx.x & (kGradCopies - 1)) * gstride;
+}
+// The zeroed arrays (one set per context, in use between these two calls), and their sum added to d_grad.
+int pdg_grad_part(pdg_context *ctx, double **part, int *gstride);
+int pdg_grad_sum(pdg_context *ctx, const double *part, int gstride, double *d_grad);
+
 // Density-screening bound of the SCF's Fock builds (full and difference): inc_cut, raised to
 // mixed_dcut in the mixed mode.
 inline double pdg_fock_dcut(const pdg_context *ctx) {

@@ -27,7 +27,7 @@ struct GradArgs {
     const double *D;
     double cx;
     int doJ;
-    double *grad;        // kGradCopies partial gradients, gstride doubles apart (grad_copy)
+    double *grad;        // kGradCopies partial gradients, gstride doubles apart (pdg_grad_copy)
     int gstride;
     int n;
     const double *dmax;  // optional (mixed mode): max |D'| per shell-pair block, nshell x nshell
@@ -36,33 +36,6 @@ struct GradArgs {
     int part;            // 0: every quartet; 1: bound >= mixed_cut (FP64); 2: bound < mixed_cut (FP32)
     double mixed_cut;
 };
-
-// Partial gradient arrays.  A molecule has only 3 natom gradient elements (about 1 KB at 42 atoms),
-// which the address hash puts in one or two L2 slices, and every quartet adds twelve values to them:
-// with one array the atomic unit of that slice was 76% busy while the FP64 pipe ran at 8% (the mean
-// over all slices was 1%).  The CTAs therefore add to kGradCopies arrays in turn, spread over the
-// slices, and grad_sum_kernel adds them up.  Gradient of a 42-atom molecule (B3LYP/6-31G*, FP64):
-// 120.0 ms with one array, 41.7 ms with the copies; a 57-atom one in the mixed mode 287 -> 108 ms.
-constexpr int kGradCopies = 128;
-__device__ __forceinline__ double *grad_copy(const GradArgs &a) {
-    return a.grad + (size_t)(blockIdx.x & (kGradCopies - 1)) * a.gstride;
-}
-
-// grad[e] += sum over the copies of part[copy][e]: 32 elements per CTA, eight threads per element.
-__global__ void __launch_bounds__(256) grad_sum_kernel(int n, int gstride, const double *__restrict__ part,
-                                                       double *__restrict__ grad) {
-    __shared__ double sh[8][33];
-    const int e = blockIdx.x * 32 + (threadIdx.x & 31), y = threadIdx.x >> 5;
-    double s = 0.0;
-    if (e < n)
-        for (int c = y; c < kGradCopies; c += 8) s += part[(size_t)c * gstride + e];
-    sh[y][threadIdx.x & 31] = s;
-    __syncthreads();
-    if (y == 0 && e < n) {
-        for (int k = 1; k < 8; ++k) s += sh[k][threadIdx.x];
-        grad[e] += s;
-    }
-}
 
 // Largest |Gamma| of a quartet from the shell-pair density maxima:
 // |4 s [D_ab D_cd - (c_x/4)(D_ac D_bd + D_ad D_bc)]| <= 4 D_AB D_CD + |c_x| (D_AC D_BD + D_AD D_BC).
@@ -314,7 +287,7 @@ __global__ void __launch_bounds__(128) eri_grad_kernel(GradArgs args) {
         }
         if (lane != 0) return;
     }
-    double *gr = grad_copy(args);
+    double *gr = pdg_grad_copy(args.grad, args.gstride);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         atomicAdd(&gr[3 * atA + k], gd[k]);
@@ -370,7 +343,7 @@ __global__ void __launch_bounds__(128) eri_grad_warp_kernel(GradArgs args) {
         }
     }
     __syncwarp();
-    double *gr = grad_copy(args);
+    double *gr = pdg_grad_copy(args.grad, args.gstride);
     double sum[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -630,7 +603,7 @@ __global__ void __launch_bounds__(128) eri_grad_group_kernel(GradArgs args) {
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) g[k] += __shfl_xor_sync(mask, g[k], o);
     if (lane == 0) {
-        double *gr = grad_copy(args);
+        double *gr = pdg_grad_copy(args.grad, args.gstride);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             atomicAdd(&gr[3 * atA + k], g[k]);
@@ -709,7 +682,38 @@ const grad_launcher grad_table[PDG_NPAIRCLASS][PDG_NPAIRCLASS] = {
 };
 #undef GL
 
+// grad[e] += sum over the copies of part[copy][e]: 32 elements per CTA, eight threads per element.
+__global__ void __launch_bounds__(256) grad_sum_kernel(int n, int gstride, const double *__restrict__ part,
+                                                       double *__restrict__ grad) {
+    __shared__ double sh[8][33];
+    const int e = blockIdx.x * 32 + (threadIdx.x & 31), y = threadIdx.x >> 5;
+    double s = 0.0;
+    if (e < n)
+        for (int c = y; c < kGradCopies; c += 8) s += part[(size_t)c * gstride + e];
+    sh[y][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (y == 0 && e < n) {
+        for (int k = 1; k < 8; ++k) s += sh[k][threadIdx.x];
+        grad[e] += s;
+    }
+}
 }  // namespace
+
+int pdg_grad_part(pdg_context *ctx, double **part, int *gstride) {
+    *gstride = (3 * ctx->natom + 15) / 16 * 16;
+    const size_t bytes = (size_t)kGradCopies * *gstride * sizeof(double);
+    *part = (double *)pdg_pool(ctx, "grad_part", bytes);
+    if (!*part) { pdg_set_error("gradient: device buffer allocation failed"); return PDG_ERR_ALLOC; }
+    PDG_CUDA(cudaMemsetAsync(*part, 0, bytes, ctx->stream));
+    return PDG_OK;
+}
+
+int pdg_grad_sum(pdg_context *ctx, const double *part, int gstride, double *d_grad) {
+    const int n3 = 3 * ctx->natom;
+    { grad_sum_kernel<<<(n3 + 31) / 32, 256, 0, ctx->stream>>>(n3, gstride, part, d_grad); pdg_count_launch(); }
+    PDG_CUDA(cudaGetLastError());
+    return PDG_OK;
+}
 
 int pdg_eri_grad(pdg_context *ctx, const double *d_D, double cx, bool doJ, double *d_grad) {
     PDG_CHECK(pdg_ensure_pairs(ctx));
@@ -726,10 +730,9 @@ int pdg_eri_grad(pdg_context *ctx, const double *d_D, double cx, bool doJ, doubl
     ctx->grad_cx = cx;
     ctx->grad_gcut = gcut;
     ProfScope prof(ctx, "eri_grad");
-    const int n3 = 3 * ctx->natom, gstride = (n3 + 15) / 16 * 16;
-    double *part = (double *)pdg_pool(ctx, "grad_part", (size_t)kGradCopies * gstride * sizeof(double));
-    if (!part) { pdg_set_error("pdg_eri_grad: device buffer allocation failed"); return PDG_ERR_ALLOC; }
-    PDG_CUDA(cudaMemsetAsync(part, 0, (size_t)kGradCopies * gstride * sizeof(double), ctx->stream));
+    int gstride = 0;
+    double *part = nullptr;
+    PDG_CHECK(pdg_grad_part(ctx, &part, &gstride));
     auto fork = std::make_unique<ClassFork>(ctx);
     for (const auto &b : ctx->blocks) {
         GradArgs a;
@@ -753,7 +756,5 @@ int pdg_eri_grad(pdg_context *ctx, const double *d_D, double cx, bool doJ, doubl
         PDG_CUDA(cudaGetLastError());
     }
     fork.reset();
-    { grad_sum_kernel<<<(n3 + 31) / 32, 256, 0, ctx->stream>>>(n3, gstride, part, d_grad); pdg_count_launch(); }
-    PDG_CUDA(cudaGetLastError());
-    return PDG_OK;
+    return pdg_grad_sum(ctx, part, gstride, d_grad);
 }

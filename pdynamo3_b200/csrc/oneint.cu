@@ -8,7 +8,7 @@
 // Raw Cartesian integrals; the
 // per-component normalisation is applied by the caller (N S N).
 #include "context.h"
-#include "rys.cuh"
+#include "md.cuh"
 
 namespace {
 
@@ -46,118 +46,103 @@ __device__ __forceinline__ void sh_xyz(const DeviceBasis &bs, int sh, double *r)
     r[0] = bs.atom_xyz[3 * at]; r[1] = bs.atom_xyz[3 * at + 1]; r[2] = bs.atom_xyz[3 * at + 2];
 }
 
-// Electron-nuclear 1D integrals for one Rys node: I[a][b], a<=IA, b<=IB.
-template <int IA, int IB>
-__device__ __forceinline__ void nuc1d(double (&I)[IA + 1][IB + 1], double g0, double c00, double b10, double AB) {
-    constexpr int L = IA + IB;
-    double G[L + 1];
-    G[0] = g0;
-    if constexpr (L > 0) {
-        G[1] = c00 * g0;
+// One warp per shell pair: its lanes take the (primitive, nucleus) terms of the attraction in turn (and the
+// primitives of overlap and kinetic energy), so that the few contracted s pairs (up to 36 primitives times
+// all nuclei, each a Boys function) do not run in one thread.  A nucleus is the ket (C|C) with one s
+// function: the Hermite sums of md.cuh with an empty ket side.  With one thread per pair and Rys rules, 96
+// atoms (25,000 s pairs: five warps per SM) took 0.89 ms for the (s|s) class,
+// 2.2 ms for all; now 0.09 ms, and 0.13 ms for the longest, (d|d).
+constexpr int OPB = 4;  // pairs (warps) per block
+
+template <int N>
+__device__ __forceinline__ void store_pair(const double (&v)[N], int nb, int oa, int ob, int n, double *__restrict__ M) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-        for (int e = 1; e < L; ++e) G[e + 1] = c00 * G[e] + e * b10 * G[e - 1];
+    for (int f = 0; f < N; ++f) {
+        const double t = warp_sum(v[f]);
+        const int ia = f / nb, jb = f % nb;
+        if (lane == 0) { M[(oa + ia) * n + ob + jb] = t; M[(ob + jb) * n + oa + ia] = t; }
     }
-    double T[L + 1][IB + 1];
-#pragma unroll
-    for (int e = 0; e <= L; ++e) T[e][0] = G[e];
-#pragma unroll
-    for (int b = 1; b <= IB; ++b)
-#pragma unroll
-        for (int a = 0; a <= L - b; ++a) T[a][b] = T[a + 1][b - 1] + AB * T[a][b - 1];
-#pragma unroll
-    for (int a = 0; a <= IA; ++a)
-#pragma unroll
-        for (int b = 0; b <= IB; ++b) I[a][b] = T[a][b];
 }
 
 template <int LA, int LB>
-__global__ void __launch_bounds__(64) oneint_kernel(PairList pl, PrimPairs pp, DeviceBasis bs, int n,
-                                                    double *__restrict__ Sm, double *__restrict__ Tm,
-                                                    double *__restrict__ Vm) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * OPB) oneint_kernel(PairList pl, PrimPairs pp, DeviceBasis bs, int n,
+                                                          double *__restrict__ Sm, double *__restrict__ Tm,
+                                                          double *__restrict__ Vm) {
+    const int t = blockIdx.x * OPB + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= pl.n) return;
     constexpr int NA = ncart(LA), NB = ncart(LB);
-    constexpr int NR = (LA + LB) / 2 + 1;
     const int A = pl.shA[t], B = pl.shB[t];
     double rA[3], rB[3];
     sh_xyz(bs, A, rA);
     sh_xyz(bs, B, rB);
-    double s[NA * NB], k[NA * NB], v[NA * NB];
-#pragma unroll
-    for (int i = 0; i < NA * NB; ++i) { s[i] = 0.0; k[i] = 0.0; v[i] = 0.0; }
-    const double AB[3] = {rA[0] - rB[0], rA[1] - rB[1], rA[2] - rB[2]};
-    for (int ip = pl.poff[t]; ip < pl.poff[t] + pl.np[t]; ++ip) {
-        const double a = pp.a[ip], b = pp.b[ip], p = a + b, r2p = 0.5 / p;
-        const double P[3] = {pp.Px[ip], pp.Py[ip], pp.Pz[ip]};
-        const double K = pp.K[ip];
-        double Sx[LA + 1][LB + 3], Sy[LA + 1][LB + 3], Sz[LA + 1][LB + 3];
-        os_overlap<LA, LB + 2>(Sx, P[0] - rA[0], P[0] - rB[0], r2p);
-        os_overlap<LA, LB + 2>(Sy, P[1] - rA[1], P[1] - rB[1], r2p);
-        os_overlap<LA, LB + 2>(Sz, P[2] - rA[2], P[2] - rB[2], r2p);
-        const double sp = PI / p;
-        const double pref = sp * sqrt(sp) * K;
-#pragma unroll
-        for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-            for (int jb = 0; jb < NB; ++jb) {
-                const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
-                const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                const double ox = Sx[ax][bx], oy = Sy[ay][by], oz = Sz[az][bz];
-                s[ia * NB + jb] += pref * ox * oy * oz;
-                k[ia * NB + jb] += pref * (kin1d<LA, LB + 2>(Sx, ax, bx, b) * oy * oz + ox * kin1d<LA, LB + 2>(Sy, ay, by, b) * oz +
-                                           ox * oy * kin1d<LA, LB + 2>(Sz, az, bz, b));
-            }
-        // electron-nuclear attraction with Gaussian nuclei: -sum_C Z_C (ab|C) with the nucleus a
-        // normalised Gaussian of exponent NUC_ZETA, i.e. a (ab|ss) integral with q = NUC_ZETA.
-        const double rhoN = p * NUC_ZETA / (p + NUC_ZETA), fz = NUC_ZETA / (p + NUC_ZETA);
-        const double vpref = NUC_PREF / (p * sqrt(p + NUC_ZETA)) * K;
-        for (int c = 0; c < bs.natom; ++c) {
-            const double Z = bs.atom_Z[c];
-            if (Z == 0.0) continue;
-            const double PC[3] = {P[0] - bs.atom_xyz[3 * c], P[1] - bs.atom_xyz[3 * c + 1], P[2] - bs.atom_xyz[3 * c + 2]};
-            const double x = rhoN * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
-            double u[NR], w[NR];
-            rys_roots<NR>(x, u, w);
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const double ur = u[r] * fz;
-                const double b10 = r2p * (1.0 - ur);
-                double Ix[LA + 1][LB + 1], Iy[LA + 1][LB + 1], Iz[LA + 1][LB + 1];
-                nuc1d<LA, LB>(Ix, 1.0, P[0] - rA[0] - ur * PC[0], b10, AB[0]);
-                nuc1d<LA, LB>(Iy, 1.0, P[1] - rA[1] - ur * PC[1], b10, AB[1]);
-                nuc1d<LA, LB>(Iz, -Z * vpref * w[r], P[2] - rA[2] - ur * PC[2], b10, AB[2]);
-#pragma unroll
-                for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-                    for (int jb = 0; jb < NB; ++jb)
-                        v[ia * NB + jb] += Ix[cart_x(LA, ia)][cart_x(LB, jb)] * Iy[cart_y(LA, ia)][cart_y(LB, jb)] *
-                                           Iz[cart_z(LA, ia)][cart_z(LB, jb)];
-            }
-        }
-    }
     const int oa = bs.sh_bf[A], ob = bs.sh_bf[B];
+    const int p0 = pl.poff[t], np = pl.np[t];
+    {
+        double s[NA * NB], k[NA * NB];
 #pragma unroll
-    for (int ia = 0; ia < NA; ++ia)
+        for (int i = 0; i < NA * NB; ++i) { s[i] = 0.0; k[i] = 0.0; }
+        for (int ip = p0 + lane; ip < p0 + np; ip += 32) {
+            const double b = pp.b[ip], p = pp.a[ip] + b, r2p = 0.5 / p;
+            const double P[3] = {pp.Px[ip], pp.Py[ip], pp.Pz[ip]};
+            double Sx[LA + 1][LB + 3], Sy[LA + 1][LB + 3], Sz[LA + 1][LB + 3];
+            os_overlap<LA, LB + 2>(Sx, P[0] - rA[0], P[0] - rB[0], r2p);
+            os_overlap<LA, LB + 2>(Sy, P[1] - rA[1], P[1] - rB[1], r2p);
+            os_overlap<LA, LB + 2>(Sz, P[2] - rA[2], P[2] - rB[2], r2p);
+            const double sp = PI / p;
+            const double pref = sp * sqrt(sp) * pp.K[ip];
 #pragma unroll
-        for (int jb = 0; jb < NB; ++jb) {
-            const int f = ia * NB + jb;
-            Sm[(oa + ia) * n + ob + jb] = s[f]; Sm[(ob + jb) * n + oa + ia] = s[f];
-            Tm[(oa + ia) * n + ob + jb] = k[f]; Tm[(ob + jb) * n + oa + ia] = k[f];
-            Vm[(oa + ia) * n + ob + jb] = v[f]; Vm[(ob + jb) * n + oa + ia] = v[f];
+            for (int ia = 0; ia < NA; ++ia)
+#pragma unroll
+                for (int jb = 0; jb < NB; ++jb) {
+                    const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
+                    const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
+                    const double ox = Sx[ax][bx], oy = Sy[ay][by], oz = Sz[az][bz];
+                    s[ia * NB + jb] += pref * ox * oy * oz;
+                    k[ia * NB + jb] += pref * (kin1d<LA, LB + 2>(Sx, ax, bx, b) * oy * oz + ox * kin1d<LA, LB + 2>(Sy, ay, by, b) * oz +
+                                               ox * oy * kin1d<LA, LB + 2>(Sz, az, bz, b));
+                }
         }
+        store_pair<NA * NB>(s, NB, oa, ob, n, Sm);
+        store_pair<NA * NB>(k, NB, oa, ob, n, Tm);
+    }
+    // electron-nuclear attraction with Gaussian nuclei: -sum_C Z_C (ab|C) with the nucleus a normalised
+    // Gaussian of exponent NUC_ZETA, i.e. a (ab|ss) integral with q = NUC_ZETA
+    double v[NA * NB];
+#pragma unroll
+    for (int i = 0; i < NA * NB; ++i) v[i] = 0.0;
+    const double zero[3] = {0.0, 0.0, 0.0};
+    for (int idx = lane; idx < np * bs.natom; idx += 32) {
+        const int j = idx / bs.natom, c = idx - j * bs.natom, ip = p0 + j;
+        const double Z = bs.atom_Z[c];
+        if (Z == 0.0) continue;
+        const double p = pp.a[ip] + pp.b[ip], rs = rsqrt(p + NUC_ZETA);
+        const double P[3] = {pp.Px[ip], pp.Py[ip], pp.Pz[ip]};
+        const double PA[3] = {P[0] - rA[0], P[1] - rA[1], P[2] - rA[2]}, PB[3] = {P[0] - rB[0], P[1] - rB[1], P[2] - rB[2]};
+        const double PC[3] = {P[0] - bs.atom_xyz[3 * c], P[1] - bs.atom_xyz[3 * c + 1], P[2] - bs.atom_xyz[3 * c + 2]};
+        md_energy<LA, LB, 0, 0, double>(p * NUC_ZETA * rs * rs, PC, -Z * NUC_PREF * rs * pp.Kp[ip], PA, PB, pp.hp[ip], zero,
+                                        zero, 0.0, v);
+    }
+    store_pair<NA * NB>(v, NB, oa, ob, n, Vm);
 }
 
 // Gradient of sum_uv [P_uv (T+V)_uv - Ws_uv S_uv] with respect to nuclear positions, where
 // P and Ws carry the component normalisation (N P N).  Ws is the energy-weighted density
 // sum_i n_i e_i C C^T.
+//
+// One warp per shell pair as above; lanes take nuclei (the smallest power of two above natom of them, up to
+// 32, the rest of the warp further primitives), so that the term on a nucleus leaves once per pair and not
+// once per primitive, and lanes add to different elements.  The blocks add to partial arrays (pdg_grad_copy).
+// One thread per pair, with three atomics per primitive and nucleus of which all lanes met on one address:
+// 2.1 ms of a 42-atom gradient, 0.35 ms of that of 2 waters.
 template <int LA, int LB>
-__global__ void __launch_bounds__(64) oneint_grad_kernel(PairList pl, PrimPairs pp, DeviceBasis bs, int n,
-                                                         const double *__restrict__ Pm, const double *__restrict__ Wm,
-                                                         double *__restrict__ grad) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * OPB) oneint_grad_kernel(PairList pl, PrimPairs pp, DeviceBasis bs, int n,
+                                                               const double *__restrict__ Pm, const double *__restrict__ Wm,
+                                                               double *__restrict__ part, int gstride) {
+    const int t = blockIdx.x * OPB + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= pl.n) return;
     constexpr int NA = ncart(LA), NB = ncart(LB);
-    constexpr int NR = (LA + LB + 1) / 2 + 1;
+    double *__restrict__ grad = pdg_grad_copy(part, gstride);
     const int A = pl.shA[t], B = pl.shB[t];
     const int atA = bs.sh_atom[A], atB = bs.sh_atom[B];
     double rA[3], rB[3];
@@ -165,28 +150,28 @@ __global__ void __launch_bounds__(64) oneint_grad_kernel(PairList pl, PrimPairs 
     sh_xyz(bs, B, rB);
     const int oa = bs.sh_bf[A], ob = bs.sh_bf[B];
     const double fac = (A == B) ? 1.0 : 2.0;
-    double Pab[NA * NB], Wab[NA * NB];
+    const int p0 = pl.poff[t], np = pl.np[t];
+    double Pab[NA * NB];
 #pragma unroll
     for (int ia = 0; ia < NA; ++ia)
 #pragma unroll
-        for (int jb = 0; jb < NB; ++jb) {
-            Pab[ia * NB + jb] = fac * Pm[(oa + ia) * n + ob + jb];
-            Wab[ia * NB + jb] = fac * Wm[(oa + ia) * n + ob + jb];
-        }
-    const double AB[3] = {rA[0] - rB[0], rA[1] - rB[1], rA[2] - rB[2]};
-    double gA[3] = {0.0, 0.0, 0.0};  // overlap + kinetic, dB = -dA
-    double gAv[3] = {0.0, 0.0, 0.0}, gBv[3] = {0.0, 0.0, 0.0};
-    for (int ip = pl.poff[t]; ip < pl.poff[t] + pl.np[t]; ++ip) {
-        const double a = pp.a[ip], b = pp.b[ip], p = a + b, r2p = 0.5 / p;
-        const double P[3] = {pp.Px[ip], pp.Py[ip], pp.Pz[ip]};
-        const double K = pp.K[ip];
-        if (atA != atB) {
+        for (int jb = 0; jb < NB; ++jb) Pab[ia * NB + jb] = fac * Pm[(oa + ia) * n + ob + jb];
+    double gA[3] = {0.0, 0.0, 0.0}, gB[3] = {0.0, 0.0, 0.0};
+    if (atA != atB) {
+        double Wab[NA * NB];
+#pragma unroll
+        for (int ia = 0; ia < NA; ++ia)
+#pragma unroll
+            for (int jb = 0; jb < NB; ++jb) Wab[ia * NB + jb] = fac * Wm[(oa + ia) * n + ob + jb];
+        for (int ip = p0 + lane; ip < p0 + np; ip += 32) {
+            const double a = pp.a[ip], b = pp.b[ip], p = a + b, r2p = 0.5 / p;
+            const double P[3] = {pp.Px[ip], pp.Py[ip], pp.Pz[ip]};
             double Sx[LA + 2][LB + 3], Sy[LA + 2][LB + 3], Sz[LA + 2][LB + 3];
             os_overlap<LA + 1, LB + 2>(Sx, P[0] - rA[0], P[0] - rB[0], r2p);
             os_overlap<LA + 1, LB + 2>(Sy, P[1] - rA[1], P[1] - rB[1], r2p);
             os_overlap<LA + 1, LB + 2>(Sz, P[2] - rA[2], P[2] - rB[2], r2p);
             const double sp = PI / p;
-            const double pref = sp * sqrt(sp) * K;
+            const double pref = sp * sqrt(sp) * pp.K[ip];
 #pragma unroll
             for (int ia = 0; ia < NA; ++ia)
 #pragma unroll
@@ -217,57 +202,46 @@ __global__ void __launch_bounds__(64) oneint_grad_kernel(PairList pl, PrimPairs 
                     gA[2] += pref * (pw * dTz - ww * dSz);
                 }
         }
-        const double rhoN = p * NUC_ZETA / (p + NUC_ZETA), fz = NUC_ZETA / (p + NUC_ZETA);
-        const double vpref = NUC_PREF / (p * sqrt(p + NUC_ZETA)) * K;
-        for (int c = 0; c < bs.natom; ++c) {
-            const double Z = bs.atom_Z[c];
-            if (Z == 0.0) continue;
-            const double PC[3] = {P[0] - bs.atom_xyz[3 * c], P[1] - bs.atom_xyz[3 * c + 1], P[2] - bs.atom_xyz[3 * c + 2]};
-            const double x = rhoN * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
-            double u[NR], w[NR];
-            rys_roots<NR>(x, u, w);
-            double cA[3] = {0.0, 0.0, 0.0}, cB[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const double ur = u[r] * fz;
-                const double b10 = r2p * (1.0 - ur);
-                double Ix[LA + 2][LB + 2], Iy[LA + 2][LB + 2], Iz[LA + 2][LB + 2];
-                nuc1d<LA + 1, LB + 1>(Ix, 1.0, P[0] - rA[0] - ur * PC[0], b10, AB[0]);
-                nuc1d<LA + 1, LB + 1>(Iy, 1.0, P[1] - rA[1] - ur * PC[1], b10, AB[1]);
-                nuc1d<LA + 1, LB + 1>(Iz, -Z * vpref * w[r], P[2] - rA[2] - ur * PC[2], b10, AB[2]);
-#pragma unroll
-                for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-                    for (int jb = 0; jb < NB; ++jb) {
-                        const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
-                        const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                        const double x0 = Ix[ax][bx], y0 = Iy[ay][by], z0 = Iz[az][bz];
-                        const double dax = 2.0 * a * Ix[ax + 1][bx] - (ax > 0 ? ax * Ix[ax > 0 ? ax - 1 : 0][bx] : 0.0);
-                        const double day = 2.0 * a * Iy[ay + 1][by] - (ay > 0 ? ay * Iy[ay > 0 ? ay - 1 : 0][by] : 0.0);
-                        const double daz = 2.0 * a * Iz[az + 1][bz] - (az > 0 ? az * Iz[az > 0 ? az - 1 : 0][bz] : 0.0);
-                        const double dbx = 2.0 * b * Ix[ax][bx + 1] - (bx > 0 ? bx * Ix[ax][bx > 0 ? bx - 1 : 0] : 0.0);
-                        const double dby = 2.0 * b * Iy[ay][by + 1] - (by > 0 ? by * Iy[ay][by > 0 ? by - 1 : 0] : 0.0);
-                        const double dbz = 2.0 * b * Iz[az][bz + 1] - (bz > 0 ? bz * Iz[az][bz > 0 ? bz - 1 : 0] : 0.0);
-                        const double pw = Pab[ia * NB + jb];
-                        cA[0] += pw * dax * y0 * z0; cA[1] += pw * x0 * day * z0; cA[2] += pw * x0 * y0 * daz;
-                        cB[0] += pw * dbx * y0 * z0; cB[1] += pw * x0 * dby * z0; cB[2] += pw * x0 * y0 * dbz;
-                    }
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                gAv[d] += cA[d];
-                gBv[d] += cB[d];
-            }
-            // translational invariance of each nuclear term: dC = -(dA + dB)
-            atomicAdd(&grad[3 * c + 0], -(cA[0] + cB[0]));
-            atomicAdd(&grad[3 * c + 1], -(cA[1] + cB[1]));
-            atomicAdd(&grad[3 * c + 2], -(cA[2] + cB[2]));
-        }
+        for (int d = 0; d < 3; ++d) gB[d] = -gA[d];  // overlap and kinetic energy: dB = -dA
     }
+    int G = 32;  // lanes over nuclei
+    while (G / 2 >= bs.natom) G /= 2;
+    const double ab[3] = {rA[0] - rB[0], rA[1] - rB[1], rA[2] - rB[2]}, zero[3] = {0.0, 0.0, 0.0};
+    for (int c = lane & (G - 1); c < bs.natom; c += G) {
+        const double Z = bs.atom_Z[c];
+        if (Z == 0.0) continue;
+        double gC[3] = {0.0, 0.0, 0.0};
+        for (int ip = p0 + lane / G; ip < p0 + np; ip += 32 / G) {
+            const double a = pp.a[ip], p = a + pp.b[ip], rs = rsqrt(p + NUC_ZETA), hp = pp.hp[ip];
+            const double P[3] = {pp.Px[ip], pp.Py[ip], pp.Pz[ip]};
+            const double PA[3] = {P[0] - rA[0], P[1] - rA[1], P[2] - rA[2]}, PB[3] = {P[0] - rB[0], P[1] - rB[1], P[2] - rB[2]};
+            const double PC[3] = {P[0] - bs.atom_xyz[3 * c], P[1] - bs.atom_xyz[3 * c + 1], P[2] - bs.atom_xyz[3 * c + 2]};
+            double dP[3], da[3], db[3], dc[3], dd[3];
+            const double e = md_gradient<LA, LB, 0, 0, double>(p * NUC_ZETA * rs * rs, PC, -Z * NUC_PREF * rs * pp.Kp[ip], PA, PB,
+                                                               hp, zero, zero, 0.0, Pab, dP, da, db, dc, dd);
+            // P = (a A + b B) / p at fixed A - B; P - A = -(b/p)(A - B), P - B = (a/p)(A - B); exp(-(a b/p) |A-B|^2);
+            // translational invariance of each nuclear term: dC = -(dA + dB) = -dP
+            const double ap = 2.0 * a * hp, bp = 1.0 - ap, ka = -2.0 * a * bp * e;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        atomicAdd(&grad[3 * atA + d], gA[d] + gAv[d]);
-        atomicAdd(&grad[3 * atB + d], -gA[d] + gBv[d]);
+            for (int k = 0; k < 3; ++k) {
+                const double ga = ap * dP[k] + ka * ab[k] - bp * da[k] + ap * db[k];
+                gA[k] += ga;
+                gB[k] += dP[k] - ga;
+                gC[k] -= dP[k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) atomicAdd(&grad[3 * c + k], gC[k]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double sa = warp_sum(gA[k]), sb = warp_sum(gB[k]);
+        if (lane == 0) {
+            atomicAdd(&grad[3 * atA + k], sa);
+            atomicAdd(&grad[3 * atB + k], sb);
+        }
     }
 }
 
@@ -275,16 +249,16 @@ constexpr int PLA[PDG_NPAIRCLASS] = {0, 1, 1, 2, 2, 2};
 constexpr int PLB[PDG_NPAIRCLASS] = {0, 0, 1, 0, 1, 2};
 
 template <int C>
-void launch_oneint(const pdg_context *ctx, double *S, double *T, double *V) {
+void launch_oneint(const pdg_context *ctx, double *S, double *T, double *V, ClassFork &fork) {
     const PairList &pl = ctx->pairs[C];
     if (pl.n == 0) return;
-    { oneint_kernel<PLA[C], PLB[C]><<<(pl.n + 63) / 64, 64, 0, ctx->stream>>>(pl, ctx->pp, ctx->dbasis, ctx->nbf, S, T, V); pdg_count_launch(); }
+    { oneint_kernel<PLA[C], PLB[C]><<<(pl.n + OPB - 1) / OPB, 32 * OPB, 0, fork.stream(pl.n)>>>(pl, ctx->pp, ctx->dbasis, ctx->nbf, S, T, V); pdg_count_launch(); }
 }
 template <int C>
-void launch_oneint_grad(const pdg_context *ctx, const double *P, const double *W, double *g) {
+void launch_oneint_grad(const pdg_context *ctx, const double *P, const double *W, double *part, int gstride, ClassFork &fork) {
     const PairList &pl = ctx->pairs[C];
     if (pl.n == 0) return;
-    { oneint_grad_kernel<PLA[C], PLB[C]><<<(pl.n + 63) / 64, 64, 0, ctx->stream>>>(pl, ctx->pp, ctx->dbasis, ctx->nbf, P, W, g); pdg_count_launch(); }
+    { oneint_grad_kernel<PLA[C], PLB[C]><<<(pl.n + OPB - 1) / OPB, 32 * OPB, 0, fork.stream(pl.n)>>>(pl, ctx->pp, ctx->dbasis, ctx->nbf, P, W, part, gstride); pdg_count_launch(); }
 }
 
 }  // namespace
@@ -296,12 +270,13 @@ int pdg_oneint(pdg_context *ctx, double *d_S, double *d_T, double *d_V) {
     PDG_CUDA(cudaMemsetAsync(d_S, 0, nn, ctx->stream));
     PDG_CUDA(cudaMemsetAsync(d_T, 0, nn, ctx->stream));
     PDG_CUDA(cudaMemsetAsync(d_V, 0, nn, ctx->stream));
-    launch_oneint<0>(ctx, d_S, d_T, d_V);
-    launch_oneint<1>(ctx, d_S, d_T, d_V);
-    launch_oneint<2>(ctx, d_S, d_T, d_V);
-    launch_oneint<3>(ctx, d_S, d_T, d_V);
-    launch_oneint<4>(ctx, d_S, d_T, d_V);
-    launch_oneint<5>(ctx, d_S, d_T, d_V);
+    ClassFork fork(ctx);
+    launch_oneint<0>(ctx, d_S, d_T, d_V, fork);
+    launch_oneint<1>(ctx, d_S, d_T, d_V, fork);
+    launch_oneint<2>(ctx, d_S, d_T, d_V, fork);
+    launch_oneint<3>(ctx, d_S, d_T, d_V, fork);
+    launch_oneint<4>(ctx, d_S, d_T, d_V, fork);
+    launch_oneint<5>(ctx, d_S, d_T, d_V, fork);
     PDG_CUDA(cudaGetLastError());
     return PDG_OK;
 }
@@ -309,12 +284,18 @@ int pdg_oneint(pdg_context *ctx, double *d_S, double *d_T, double *d_V) {
 int pdg_oneint_grad(pdg_context *ctx, const double *d_P, const double *d_W, double *d_grad) {
     PDG_CHECK(pdg_ensure_pairs(ctx));
     ProfScope prof(ctx, "oneint_grad");
-    launch_oneint_grad<0>(ctx, d_P, d_W, d_grad);
-    launch_oneint_grad<1>(ctx, d_P, d_W, d_grad);
-    launch_oneint_grad<2>(ctx, d_P, d_W, d_grad);
-    launch_oneint_grad<3>(ctx, d_P, d_W, d_grad);
-    launch_oneint_grad<4>(ctx, d_P, d_W, d_grad);
-    launch_oneint_grad<5>(ctx, d_P, d_W, d_grad);
+    int gstride = 0;
+    double *part = nullptr;
+    PDG_CHECK(pdg_grad_part(ctx, &part, &gstride));
+    {
+        ClassFork fork(ctx);
+        launch_oneint_grad<0>(ctx, d_P, d_W, part, gstride, fork);
+        launch_oneint_grad<1>(ctx, d_P, d_W, part, gstride, fork);
+        launch_oneint_grad<2>(ctx, d_P, d_W, part, gstride, fork);
+        launch_oneint_grad<3>(ctx, d_P, d_W, part, gstride, fork);
+        launch_oneint_grad<4>(ctx, d_P, d_W, part, gstride, fork);
+        launch_oneint_grad<5>(ctx, d_P, d_W, part, gstride, fork);
+    }
     PDG_CUDA(cudaGetLastError());
-    return PDG_OK;
+    return pdg_grad_sum(ctx, part, gstride, d_grad);
 }
