@@ -106,7 +106,7 @@ __device__ __forceinline__ double pasc_ds(double nu) {
 // nearest to its first point), so that all lanes read the same elements.
 constexpr double CELL_REL = 1.0e-20;
 constexpr int CELL_U = 4;    // factors formed between two tests of the cut: their loads and series overlap
-constexpr int CELL_M = 16;   // distances of the first atoms of the order kept in shared memory
+constexpr int CELL_M = 24;   // distances of the first atoms of the order kept in shared memory
 
 __device__ __forceinline__ double point_dist(const double *__restrict__ xyz, int i, double px, double py, double pz) {
     const double dx = xyz[3 * i] - px, dy = xyz[3 * i + 1] - py, dz = xyz[3 * i + 2] - pz;
@@ -158,6 +158,36 @@ __device__ __forceinline__ void cell_row(int k, double Rk, int n, const int *__r
             if (s[q] < mn) { rest *= mn; mn = s[q]; } else rest *= s[q];
         }
         if (fabs(rest) < tiny) break;
+    }
+}
+
+// CELL_T cell functions at a time, |A| <= tiny cut: the products A of the rows k[] at distances Rk[], over the
+// atoms in the order ord, until all of them are below tiny (0: never).  One distance per atom serves all
+// rows (past the first CELL_M it is a square root, more work than the factor itself), and the rows' series
+// run side by side.  Weights of 1.35 M candidates of a 96-atom cluster 15.5 -> 12.7 ms.
+constexpr int CELL_T = 4;
+template <typename Dist>
+__device__ __forceinline__ void cell_rows(const int (&k)[CELL_T], const double (&Rk)[CELL_T], int n, const int *__restrict__ ord,
+                                          const double2 *__restrict__ pij, Dist dist, double tiny, double (&A)[CELL_T]) {
+    const double2 *row[CELL_T];
+#pragma unroll
+    for (int q = 0; q < CELL_T; ++q) {
+        row[q] = pij + (size_t)k[q] * n;
+        A[q] = 1.0;
+    }
+    for (int r = 0; r < n; ++r) {
+        const int j = ord[r];
+        const double Rj = dist(r, j);
+        double big = 0.0;
+#pragma unroll
+        for (int q = 0; q < CELL_T; ++q) {
+            const double2 p = row[q][j];
+            const double mu = (Rk[q] - Rj) * p.x;
+            const double v = pasc_s(mu + p.y * (1.0 - mu * mu));
+            if (j != k[q]) A[q] *= v;
+            big = fmax(big, fabs(A[q]));
+        }
+        if (big < tiny) break;
     }
 }
 
@@ -1077,15 +1107,36 @@ __global__ void __launch_bounds__(128) grid_candidates_kernel(
     double *R = &cR[0][threadIdx.x];
     for (int i = 0; i < min(natom, CELL_M); ++i) R[i * 128] = point_dist(xyz, ord[i], px, py, pz);
     const auto dist = [&](int rk, int j) { return rk < CELL_M ? R[rk * 128] : point_dist(xyz, j, px, py, pz); };
-    double mn, rest;
-    cell_row(g, point_dist(xyz, g, px, py, pz), natom, ord, pij + (size_t)g * natom, dist, 0.0, mn, rest);
-    const double pg = mn * rest;
-    double sum = pg;
-    for (int rk = 0; rk < natom; ++rk) {
-        const int k = ord[rk];
-        if (k == g) continue;
-        cell_row(k, dist(rk, k), natom, ord, pij + (size_t)k * natom, dist, CELL_REL * sum, mn, rest);
-        sum += mn * rest;
+    // the own atom's row with the first of the order, in full; then the others by rank, cut
+    double pg, sum;
+    {
+        int k[CELL_T];
+        double Rk[CELL_T], A[CELL_T];
+        k[0] = g;
+        Rk[0] = point_dist(xyz, g, px, py, pz);
+#pragma unroll
+        for (int q = 1; q < CELL_T; ++q) {
+            k[q] = ord[min(q - 1, natom - 1)];
+            Rk[q] = dist(min(q - 1, natom - 1), k[q]);
+        }
+        cell_rows(k, Rk, natom, ord, pij, dist, 0.0, A);
+        pg = sum = A[0];
+#pragma unroll
+        for (int q = 1; q < CELL_T; ++q)
+            if (q - 1 < natom && k[q] != g) sum += A[q];
+    }
+    for (int rk = CELL_T - 1; rk < natom; rk += CELL_T) {
+        int k[CELL_T];
+        double Rk[CELL_T], A[CELL_T];
+#pragma unroll
+        for (int q = 0; q < CELL_T; ++q) {
+            k[q] = ord[min(rk + q, natom - 1)];
+            Rk[q] = dist(min(rk + q, natom - 1), k[q]);
+        }
+        cell_rows(k, Rk, natom, ord, pij, dist, CELL_REL * sum, A);
+#pragma unroll
+        for (int q = 0; q < CELL_T; ++q)
+            if (rk + q < natom && k[q] != g) sum += A[q];
     }
     const double w = wraw * (pg / sum);
     if (!valid) return;
