@@ -257,13 +257,40 @@ __global__ void basis_values_kernel(int nblk, const int *__restrict__ bstart, co
         px = pts[4 * q]; py = pts[4 * q + 1]; pz = pts[4 * q + 2];
     }
     double *V = bval + voff[b];
+    int cur = -1, l = 0, f0 = 0;
+    double dx = 0.0, dy = 0.0, dz = 0.0, r0 = 0.0, r1 = 0.0;
     for (int i = 0; i < nf; ++i) {
-        double o[4] = {0, 0, 0, 0};
-        if (p < np) basis_eval<1>(bs, fun[foff[b] + i], px, py, pz, o);
-        V[(0 * nf + i) * BLK + p] = o[0];
-        V[(1 * nf + i) * BLK + p] = o[1];
-        V[(2 * nf + i) * BLK + p] = o[2];
-        V[(3 * nf + i) * BLK + p] = o[3];
+        const int f = fun[foff[b] + i], sh = bs.bf_shell[f];
+        if (sh != cur) {  // the radial sums of a shell, for all its functions
+            cur = sh;
+            l = bs.sh_l[sh];
+            f0 = bs.sh_bf[sh];
+            const int at = bs.sh_atom[sh], k0 = bs.sh_poff[sh], k1 = k0 + bs.sh_np[sh];
+            dx = px - bs.atom_xyz[3 * at]; dy = py - bs.atom_xyz[3 * at + 1]; dz = pz - bs.atom_xyz[3 * at + 2];
+            const double d2 = dx * dx + dy * dy + dz * dz;
+            r0 = r1 = 0.0;
+            for (int k = k0; k < k1; ++k) {
+                const double a = bs.prim_exp[k], ar2 = a * d2;
+                if (ar2 > 740.0) continue;
+                const double g = bs.prim_coef[k] * exp(-ar2);
+                r0 += g;
+                r1 -= 2.0 * a * g;
+            }
+        }
+        const int c = f - f0;
+        const int lx = l == 0 ? 0 : l == 1 ? c == 0 : cart_x(2, c), ly = l == 0 ? 0 : l == 1 ? c == 1 : cart_y(2, c);
+        const int lz = l - lx - ly;
+        const double X = lx == 0 ? 1.0 : lx == 1 ? dx : dx * dx, Y = ly == 0 ? 1.0 : ly == 1 ? dy : dy * dy;
+        const double Z = lz == 0 ? 1.0 : lz == 1 ? dz : dz * dz;
+        // d/dx of x^l exp: l x^(l-1) r0 + x^(l+1) r1
+        const double X1 = X * dx * r1 + (lx == 0 ? 0.0 : lx == 1 ? r0 : 2.0 * dx * r0);
+        const double Y1 = Y * dy * r1 + (ly == 0 ? 0.0 : ly == 1 ? r0 : 2.0 * dy * r0);
+        const double Z1 = Z * dz * r1 + (lz == 0 ? 0.0 : lz == 1 ? r0 : 2.0 * dz * r0);
+        const bool in = p < np;
+        V[(0 * nf + i) * BLK + p] = in ? X * Y * Z * r0 : 0.0;
+        V[(1 * nf + i) * BLK + p] = in ? X1 * Y * Z : 0.0;
+        V[(2 * nf + i) * BLK + p] = in ? X * Y1 * Z : 0.0;
+        V[(3 * nf + i) * BLK + p] = in ? X * Y * Z1 : 0.0;
     }
 }
 
@@ -1211,9 +1238,46 @@ __global__ void gather_atom_pos_kernel(int natom, const long long *__restrict__ 
     out[a] = (a < natom && aoff[a] < ncand) ? pos[aoff[a]] : total;
 }
 
+// Functions (bits) of a split shell of angular momentum L whose largest |phi| over the np points exceeds
+// tol.  One warp: 32 points at a time, until every function has been found.
+template <int L>
+__device__ __forceinline__ unsigned shell_hits(const DeviceBasis &bs, int s, int np, const double (&pt)[3][BLK], double tol) {
+    constexpr int NF = ncart(L);
+    const int at = bs.sh_atom[s], f0 = bs.sh_bf[s], k0 = bs.sh_poff[s], k1 = k0 + bs.sh_np[s], lane = threadIdx.x & 31;
+    const double x = bs.atom_xyz[3 * at], y = bs.atom_xyz[3 * at + 1], z = bs.atom_xyz[3 * at + 2];
+    unsigned hit = 0;
+    for (int base = 0; base < np && hit != (1u << NF) - 1u; base += 32) {
+        const int p = min(base + lane, np - 1);
+        const double dx = pt[0][p] - x, dy = pt[1][p] - y, dz = pt[2][p] - z;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        double v[NF];
+#pragma unroll
+        for (int i = 0; i < NF; ++i) v[i] = 0.0;
+        for (int k = k0; k < k1; ++k) {
+            const double ar2 = bs.prim_exp[k] * r2;
+            if (ar2 > 740.0) continue;
+            const double g = bs.prim_coef[k] * exp(-ar2);
+#pragma unroll
+            for (int i = 0; i < NF; ++i) {
+                const double X = cart_x(L, i) == 0 ? 1.0 : cart_x(L, i) == 1 ? dx : dx * dx;
+                const double Y = cart_y(L, i) == 0 ? 1.0 : cart_y(L, i) == 1 ? dy : dy * dy;
+                const double Z = cart_z(L, i) == 0 ? 1.0 : cart_z(L, i) == 1 ? dz : dz * dz;
+                v[i] += g * X * Y * Z;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < NF; ++i)
+            if (__any_sync(0xffffffffu, fabs(v[i] * bs.bf_norm[f0 + i]) > tol)) hit |= 1u << i;
+    }
+    return hit;
+}
+
 // Per block: centroid and radius of its points, distance screen of every split shell, and for the
-// surviving shells the largest |phi| of each function over the points; mask[b][f] = 1 above the
-// reference's value tolerance (GridFunctionDataBlock_FilterValues, GridFunctionDataBlock.c:130).
+// surviving shells the functions with a value above the reference's tolerance on any point
+// (GridFunctionDataBlock_FilterValues, GridFunctionDataBlock.c:130); mask[b][f] = 1 for these.  The warps
+// share out the shells: a shell's exponentials serve all its functions, there is no barrier per function,
+// and most shells are settled by their first 32 points.
 __global__ void __launch_bounds__(BLK) block_screen_kernel(int nblk, const int *__restrict__ bstart,
                                                            const int *__restrict__ bcount, const double *__restrict__ pts,
                                                            const double *__restrict__ shell_rad, DeviceBasis bs,
@@ -1222,11 +1286,13 @@ __global__ void __launch_bounds__(BLK) block_screen_kernel(int nblk, const int *
     const int np = bcount[b];
     __shared__ double red[4][BLK / 32];
     __shared__ double cen[4];
+    __shared__ double pt[3][BLK];
     double px = 0, py = 0, pz = 0;
     if (p < np) {
         const long long q = (long long)bstart[b] + p;
         px = pts[4 * q]; py = pts[4 * q + 1]; pz = pts[4 * q + 2];
     }
+    pt[0][p] = px; pt[1][p] = py; pt[2][p] = pz;
     double sx = px, sy = py, sz = pz;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1254,32 +1320,16 @@ __global__ void __launch_bounds__(BLK) block_screen_kernel(int nblk, const int *
     double rad = red[3][0];
     for (int k = 1; k < BLK / 32; ++k) rad = fmax(rad, red[3][k]);
     unsigned char *mb = mask + (long long)b * bs.nbf;
-    for (int s = 0; s < bs.nshell; ++s) {
-        const int at = bs.sh_atom[s], nf = ncart(bs.sh_l[s]), f0 = bs.sh_bf[s];
+    for (int s = w; s < bs.nshell; s += BLK / 32) {
+        const int at = bs.sh_atom[s], l = bs.sh_l[s], nf = ncart(l), f0 = bs.sh_bf[s];
         const double dx = bs.atom_xyz[3 * at] - cen[0], dy = bs.atom_xyz[3 * at + 1] - cen[1], dz = bs.atom_xyz[3 * at + 2] - cen[2];
-        if (sqrt(dx * dx + dy * dy + dz * dz) - rad >= shell_rad[s]) {
-            if (p < nf) mb[f0 + p] = 0;
-            continue;
+        unsigned hit = 0;
+        if (sqrt(dx * dx + dy * dy + dz * dz) - rad < shell_rad[s]) {
+            if (l == 0) hit = shell_hits<0>(bs, s, np, pt, bf_tol);
+            else if (l == 1) hit = shell_hits<1>(bs, s, np, pt, bf_tol);
+            else hit = shell_hits<2>(bs, s, np, pt, bf_tol);
         }
-        for (int i = 0; i < nf; ++i) {
-            const int f = f0 + i;
-            double v = 0.0;
-            if (p < np) {
-                double o[1];
-                basis_eval<0>(bs, f, px, py, pz, o);
-                v = fabs(o[0] * bs.bf_norm[f]);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-            __syncthreads();  // red[0] reuse
-            if (lane == 0) red[0][w] = v;
-            __syncthreads();
-            if (p == 0) {
-                double m = red[0][0];
-                for (int k = 1; k < BLK / 32; ++k) m = fmax(m, red[0][k]);
-                mb[f] = m > bf_tol ? 1 : 0;
-            }
-        }
+        if (lane < nf) mb[f0 + lane] = hit >> lane & 1u;
     }
 }
 
