@@ -191,58 +191,7 @@ __device__ __forceinline__ void cell_rows(const int (&k)[CELL_T], const double (
     }
 }
 
-// Basis function (raw Cartesian) value and derivatives up to second order at a point.
-// out: 0 value, 1-3 x y z, 4-9 xx xy xz yy yz zz.
-template <int ORDER>
-__device__ __forceinline__ void basis_eval(const DeviceBasis &bs, int f, double px, double py, double pz, double *out) {
-    const int sh = bs.bf_shell[f];
-    const int l = bs.sh_l[sh];
-    const int comp = f - bs.sh_bf[sh];
-    int lx, ly, lz;
-    if (l == 0) { lx = ly = lz = 0; }
-    else if (l == 1) { lx = comp == 0; ly = comp == 1; lz = comp == 2; }
-    else { lx = cart_x(2, comp); ly = cart_y(2, comp); lz = cart_z(2, comp); }
-    const int at = bs.sh_atom[sh];
-    const double dx = px - bs.atom_xyz[3 * at], dy = py - bs.atom_xyz[3 * at + 1], dz = pz - bs.atom_xyz[3 * at + 2];
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    // powers
-    auto pw = [](double x, int n) { return n == 0 ? 1.0 : n == 1 ? x : n == 2 ? x * x : n == 3 ? x * x * x : x * x * x * x; };
-    const double X0 = pw(dx, lx), Y0 = pw(dy, ly), Z0 = pw(dz, lz);
-    const double Xm = lx >= 1 ? pw(dx, lx - 1) : 0.0, Ym = ly >= 1 ? pw(dy, ly - 1) : 0.0, Zm = lz >= 1 ? pw(dz, lz - 1) : 0.0;
-    const double Xmm = lx >= 2 ? pw(dx, lx - 2) : 0.0, Ymm = ly >= 2 ? pw(dy, ly - 2) : 0.0, Zmm = lz >= 2 ? pw(dz, lz - 2) : 0.0;
-    double v = 0, vx = 0, vy = 0, vz = 0, vxx = 0, vxy = 0, vxz = 0, vyy = 0, vyz = 0, vzz = 0;
-    const int p0 = bs.sh_poff[sh], np = bs.sh_np[sh];
-    for (int k = p0; k < p0 + np; ++k) {
-        const double a = bs.prim_exp[k];
-        const double ar2 = a * r2;
-        if (ar2 > 740.0) continue;
-        const double g = bs.prim_coef[k] * exp(-ar2);
-        v += g * X0 * Y0 * Z0;
-        if (ORDER >= 1) {
-            const double ta = 2.0 * a;
-            const double X1 = lx * Xm - ta * X0 * dx, Y1 = ly * Ym - ta * Y0 * dy, Z1 = lz * Zm - ta * Z0 * dz;
-            vx += g * X1 * Y0 * Z0;
-            vy += g * X0 * Y1 * Z0;
-            vz += g * X0 * Y0 * Z1;
-            if (ORDER >= 2) {
-                const double X2 = lx * (lx - 1) * Xmm - ta * (2 * lx + 1) * X0 + ta * ta * X0 * dx * dx;
-                const double Y2 = ly * (ly - 1) * Ymm - ta * (2 * ly + 1) * Y0 + ta * ta * Y0 * dy * dy;
-                const double Z2 = lz * (lz - 1) * Zmm - ta * (2 * lz + 1) * Z0 + ta * ta * Z0 * dz * dz;
-                vxx += g * X2 * Y0 * Z0;
-                vyy += g * X0 * Y2 * Z0;
-                vzz += g * X0 * Y0 * Z2;
-                vxy += g * X1 * Y1 * Z0;
-                vxz += g * X1 * Y0 * Z1;
-                vyz += g * X0 * Y1 * Z1;
-            }
-        }
-    }
-    out[0] = v;
-    if (ORDER >= 1) { out[1] = vx; out[2] = vy; out[3] = vz; }
-    if (ORDER >= 2) { out[4] = vxx; out[5] = vxy; out[6] = vxz; out[7] = vyy; out[8] = vyz; out[9] = vzz; }
-}
-
-// Resident basis values [4][nfun][128] per block.
+// Resident basis values [4][nfun][128] per block: value and gradient of each kept function (raw Cartesian).
 __global__ void basis_values_kernel(int nblk, const int *__restrict__ bstart, const int *__restrict__ bcount,
                                     const long long *__restrict__ foff, const int *__restrict__ fun,
                                     const long long *__restrict__ voff, const double *__restrict__ pts, DeviceBasis bs,
@@ -782,19 +731,51 @@ __global__ void __launch_bounds__(XT, 1) xc_grad_dmma_kernel(GradArgs a) {
         for (int i = 0; i < 4; ++i) {
             const int mu = m0 + wm * 32 + 8 * i + g;
             if (mu >= nf) continue;
-            const int f = sfun[mu];
+            const int f = sfun[mu], sh = a.bs.bf_shell[f], l = a.bs.sh_l[sh], cc = f - a.bs.sh_bf[sh], at = a.bs.sh_atom[sh];
+            const int lx = l == 0 ? 0 : l == 1 ? cc == 0 : cart_x(2, cc), ly = l == 0 ? 0 : l == 1 ? cc == 1 : cart_y(2, cc);
+            const int lz = l - lx - ly;
+            const double x0 = a.bs.atom_xyz[3 * at], y0 = a.bs.atom_xyz[3 * at + 1], z0 = a.bs.atom_xyz[3 * at + 2];
+            // phi = A(x, y, z) r0 with the monomial A and the radial sums r0 = sum g, r1 = -sum 2 a g,
+            // r2 = sum 4 a^2 g of the lane's eight points, the exponentials of which run side by side
+            double d2[8], r0[8], r1[8], r2[8];
 #pragma unroll
             for (int jc = 0; jc < 8; ++jc) {
-                const int j = jc >> 1, c = jc & 1;
-                const int p = wp * 32 + 8 * j + 2 * q + c;
+                const int p = wp * 32 + 8 * (jc >> 1) + 2 * q + (jc & 1);
+                const double dx = S.pt[0][p] - x0, dy = S.pt[1][p] - y0, dz = S.pt[2][p] - z0;
+                d2[jc] = dx * dx + dy * dy + dz * dz;
+                r0[jc] = r1[jc] = r2[jc] = 0.0;
+            }
+            for (int k = a.bs.sh_poff[sh], k1 = k + a.bs.sh_np[sh]; k < k1; ++k) {
+                const double ea = a.bs.prim_exp[k], co = a.bs.prim_coef[k], m2a = -2.0 * ea;
+#pragma unroll
+                for (int jc = 0; jc < 8; ++jc) {
+                    const double ar2 = ea * d2[jc];
+                    const double e = ar2 > 740.0 ? 0.0 : co * exp(-ar2), e1 = m2a * e;
+                    r0[jc] += e;
+                    r1[jc] += e1;
+                    r2[jc] = fma(m2a, e1, r2[jc]);
+                }
+            }
+#pragma unroll
+            for (int jc = 0; jc < 8; ++jc) {
+                const int p = wp * 32 + 8 * (jc >> 1) + 2 * q + (jc & 1);
                 if (p >= np) continue;
-                const double X = ax[i][j][c];
+                const double dx = S.pt[0][p] - x0, dy = S.pt[1][p] - y0, dz = S.pt[2][p] - z0;
                 const double ca = S.cf[0][p], cx = S.cf[1][p], cy = S.cf[2][p], cz = S.cf[3][p];
-                double h[10];
-                basis_eval<2>(a.bs, f, S.pt[0][p], S.pt[1][p], S.pt[2][p], h);
-                gs[i][0] += (ca * h[1] + cx * h[4] + cy * h[5] + cz * h[6]) * X;
-                gs[i][1] += (ca * h[2] + cx * h[5] + cy * h[7] + cz * h[8]) * X;
-                gs[i][2] += (ca * h[3] + cx * h[6] + cy * h[8] + cz * h[9]) * X;
+                const double X = lx == 0 ? 1.0 : lx == 1 ? dx : dx * dx, Y = ly == 0 ? 1.0 : ly == 1 ? dy : dy * dy;
+                const double Z = lz == 0 ? 1.0 : lz == 1 ? dz : dz * dz;
+                const double Xp = lx == 0 ? 0.0 : lx == 1 ? 1.0 : 2.0 * dx, Yp = ly == 0 ? 0.0 : ly == 1 ? 1.0 : 2.0 * dy;
+                const double Zp = lz == 0 ? 0.0 : lz == 1 ? 1.0 : 2.0 * dz;
+                const double A = X * Y * Z, Ax = Xp * Y * Z, Ay = X * Yp * Z, Az = X * Y * Zp;
+                const double Axx = lx == 2 ? 2.0 * Y * Z : 0.0, Ayy = ly == 2 ? 2.0 * X * Z : 0.0, Azz = lz == 2 ? 2.0 * X * Y : 0.0;
+                const double Axy = Xp * Yp * Z, Axz = Xp * Y * Zp, Ayz = X * Yp * Zp;
+                // ca d_d phi + sum_b c_b d_b d_d phi
+                const double cd = cx * dx + cy * dy + cz * dz, cA = cx * Ax + cy * Ay + cz * Az;
+                const double u = ca * r0[jc] + cd * r1[jc], v = (ca * A + cA) * r1[jc] + A * cd * r2[jc], w = A * r1[jc];
+                const double xx = ax[i][jc >> 1][jc & 1];
+                gs[i][0] += (Ax * u + dx * v + cx * w + (cx * Axx + cy * Axy + cz * Axz) * r0[jc]) * xx;
+                gs[i][1] += (Ay * u + dy * v + cy * w + (cx * Axy + cy * Ayy + cz * Ayz) * r0[jc]) * xx;
+                gs[i][2] += (Az * u + dz * v + cz * w + (cx * Axz + cy * Ayz + cz * Azz) * r0[jc]) * xx;
             }
         }
 #pragma unroll
