@@ -22,6 +22,8 @@ int pdg_out_to_cart(pdg_context *ctx, const double *Mo, double *Mc);
 int pdg_fock2_scf(pdg_context *ctx, double cx, bool doJ, double *d_F2);
 int pdg_store_packed(pdg_context *ctx, const double *d_full_out, double *packed_host);
 int pdg_gradients_device(pdg_context *ctx, double cx, bool doJ, std::vector<double> &g);
+bool pdg_purify_fits(int m);
+int pdg_purify_cluster(pdg_context *ctx, int m, double *d_Q, double *d_status);
 int pdg_oneint_grad(pdg_context *ctx, const double *d_P, const double *d_W, double *d_grad);
 int pdg_eri_grad(pdg_context *ctx, const double *d_D, double cx, bool doJ, double *d_grad);
 int pdg_shell_pair_dmax(pdg_context *ctx, const double *d_D, double *d_dmax);
@@ -239,7 +241,8 @@ int diagonalise(pdg_context *ctx, ScfState &st, const double *F) {
 //   P <- ((1+c) P^2 - P^3) / c               (c >= 1/2)
 //   P <- ((1-2c) P + (1+c) P^2 - P^3) / (1-c) (c <  1/2)
 // keeps the trace at nocc and converges to that projector; it needs only GEMMs, where a dense
-// eigensolver of this size is bound by its serial tridiagonalisation.
+// eigensolver of this size is bound by its serial tridiagonalisation.  Small matrices take all steps in one
+// launch (purify.cu).
 
 // Gershgorin discs, one warp per row: rows[i] = F_ii - sum_j |F_ij|, rows[m + i] = F_ii + sum_j |F_ij|
 // (j != i), rows[2m + i] = F_ii.
@@ -338,7 +341,14 @@ int purify_density(pdg_context *ctx, ScfState &st, const double *F, int nocc, do
     const int grid = (int)std::min<long long>(32, (n + 255) / 256);
     { purify_init_kernel<<<grid, 256, 0, ctx->stream>>>(m, st.T2, rows, nocc, Q); pdg_count_launch(); }
     bool done = false;
-    for (int it = 0; it < 120 && !done; ++it) {
+    const bool cluster = pdg_purify_fits(m);
+    if (cluster) {
+        PDG_CHECK(pdg_purify_cluster(ctx, m, Q, sc + 3));
+        double t;
+        PDG_CHECK(fetch(ctx, sc + 3, 1, &t));
+        done = std::fabs(t) < 1e-12;
+    }
+    for (int it = 0; it < 120 && !done && !cluster; ++it) {
         PDG_CHECK(gemm(ctx, CUBLAS_OP_N, CUBLAS_OP_N, m, m, m, 1.0, Q, m, Q, m, 0.0, Q2, m));
         PDG_CHECK(gemm(ctx, CUBLAS_OP_N, CUBLAS_OP_N, m, m, m, 1.0, Q2, m, Q, m, 0.0, Q3, m));
         { purify_step_kernel<<<grid, 256, 0, ctx->stream>>>(m, Q, Q2, Q3, Qn, sc + 3); pdg_count_launch(); }
