@@ -71,7 +71,7 @@ struct pdg_context {
     std::vector<int> bucket_start[PDG_NPAIRCLASS]; // per class: first pair of each bucket (PDG_NBUCKET + 1)
     std::vector<int> bucket_group[PDG_NPAIRCLASS]; // per class: first ket group of each bucket
     std::vector<int> hostPoff[PDG_NPAIRCLASS], hostNp[PDG_NPAIRCLASS];  // sorted pair -> primitive pairs
-    std::vector<double> hostArg;                                        // primitive-pair exponent arguments
+    std::vector<double> hostArg;                                        // primitive-pair exponent arguments (read back for pdg_work_estimate)
     PrimPairs pp{};
     int npp = 0;
     double qmax[PDG_NPAIRCLASS]{};
@@ -247,6 +247,13 @@ inline long long pdg_fill_work(WorkList &w, const QuartetBlock &b, const int (&l
         }
     }
     return cta;
+}
+
+// Threads of that launch.
+inline long long pdg_work_threads(const QuartetBlock &b, const int (&lanes)[PDG_NBUCKET]) {
+    long long n = 0;
+    for (int k = 0; k < b.nsub; ++k) n += b.sub[k].total * lanes[b.sub[k].bucket];
+    return n;
 }
 
 // The same for the warp-per-bra kernels: one warp per (bra pair, ket group) item, four to a CTA.

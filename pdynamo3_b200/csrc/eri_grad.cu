@@ -628,8 +628,12 @@ constexpr int PLA[PDG_NPAIRCLASS] = {0, 1, 1, 2, 2, 2};
 constexpr int PLB[PDG_NPAIRCLASS] = {0, 0, 1, 0, 1, 2};
 
 // Lanes per quartet of the one-thread gradient form by ket bucket: the buckets with many primitive
-// pairs split their primitive quartets.
-constexpr int kGradLanes[PDG_NBUCKET] = {1, 1, 2, 4, 4};
+// pairs split their primitive quartets.  A list of few quartets takes the rows of more lanes while its
+// threads stay below kGradLaneThreads, about those that fit the chip at the kernels' registers: the launch
+// then lasts as long as its longest quartet, 0.6 ms for (pp|pp) at two lanes.
+constexpr int kNGradLanes = 4;
+constexpr int kGradLanes[kNGradLanes][PDG_NBUCKET] = {{1, 1, 2, 4, 4}, {1, 2, 4, 8, 8}, {2, 4, 8, 16, 16}, {4, 8, 16, 32, 32}};
+constexpr long long kGradLaneThreads = 148 * 256;
 // Lists of at least this many (bra, ket group) items take the warp-per-bra form: every SM then has its
 // resident warps (8 to 16 at these register counts) more than once over; below it one lane per quartet
 // would leave SMs idle.
@@ -660,7 +664,9 @@ void launch_grad_t(const GradArgs &a0, const QuartetBlock &b, cudaStream_t st) {
             { eri_grad_warp_kernel<LA, LB, LC, LD, float><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
             return;
         }
-        const long long blocks = pdg_fill_work(a.work, b, kGradLanes);
+        int v = 0;
+        while (v + 1 < kNGradLanes && pdg_work_threads(b, kGradLanes[v + 1]) <= kGradLaneThreads) ++v;
+        const long long blocks = pdg_fill_work(a.work, b, kGradLanes[v]);
         // mixed mode: the quartets above the mixed cut in FP64, the rest in FP32
         if (mixed) a.part = 1;
         { eri_grad_kernel<LA, LB, LC, LD, double><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }

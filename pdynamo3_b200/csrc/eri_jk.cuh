@@ -66,8 +66,8 @@ __host__ __device__ constexpr int jk_group(int la, int lb, int lc, int ld) {
          : 0;
 }
 
-// One-quartet-per-thread form: the small component blocks split their primitive quartets over lanes,
-// more lanes for the ket buckets with more primitive pairs.
+// The classes of small component blocks (up to 36) split their primitive quartets over lanes, more lanes
+// for the ket buckets with more primitive pairs; the wider blocks only in short lists (kWideLanes).
 __host__ __device__ constexpr bool jk_split(int la, int lb, int lc, int ld) {
     return ncart(la) * ncart(lb) * ncart(lc) * ncart(ld) <= 36;
 }
@@ -86,7 +86,14 @@ constexpr int kDefaultLanesV[PDG_NPAIRCLASS][PDG_NPAIRCLASS] = {
 // primitives of a quartet, so a shorter list leaves the chip waiting for its longest quartets and keeps
 // several lanes per quartet (4 waters: 1.20 ms so, 1.36 ms with the line at 2368 items).
 constexpr long long kWarpItems = 8192;
-constexpr int kOneLane[PDG_NBUCKET] = {1, 1, 1, 1, 1};
+// A list of few quartets takes the tables of more lanes while its threads stay below kLaneThreads, one to
+// two times those that fit the chip at the kernels' registers: the launch then lasts as long as its longest
+// quartet, and one lane takes 0.2 ms for the 81 primitive quartets of a (pp|pp) one.  Lanes beyond that
+// only repeat the quartets' preambles.  The same for the classes of wide blocks, from one lane per
+// quartet and at half the threads (255 registers).
+constexpr long long kLaneThreads = 148 * 1024;
+constexpr int kNWide = 4;
+constexpr int kWideLanes[kNWide][PDG_NBUCKET] = {{1, 1, 1, 1, 1}, {1, 2, 2, 2, 2}, {2, 4, 4, 4, 4}, {4, 8, 8, 8, 8}};
 
 }  // namespace
 
@@ -295,18 +302,18 @@ __device__ __forceinline__ JKScreen jk_screen(const JKArgs &args, int ib, int ik
     return r;
 }
 
-// One shell quartet per P lanes (SPLIT: P = the bucket's lane count, 1 to 8; else 1): the lanes split
+// One shell quartet per P lanes (the bucket's lane count, 1 to 32): the lanes split
 // the primitive quartets and add their blocks with shuffles; the first lanes digest, one the J part
 // and up to two the K parts (rows of a, rows of b), as independent streams of loads and atomics that
 // the warp scheduler interleaves.  Splitting keeps more primitive loads in flight for the contracted
 // s/p classes (up to 6 x 6 primitive pairs per shell pair), whose one-lane loops are bound by load
 // latency; the ket buckets give the quartets of a warp the same primitive count.
-template <int LA, int LB, int LC, int LD, bool DOJ, bool DOK, typename T = double, bool SPLIT = false>
+template <int LA, int LB, int LC, int LD, bool DOJ, bool DOK, typename T>
 __global__ void __launch_bounds__(128) eri_jk_kernel(JKArgs args) {
     const WorkSub ws = pick_sub(args.work);
-    const int P = SPLIT ? ws.lanes : 1;
+    const int P = ws.lanes;
     const long long t = ((long long)blockIdx.x - ws.cta0) * blockDim.x / P + (long long)(threadIdx.x / P);
-    const int lane = SPLIT ? (int)(threadIdx.x & (P - 1)) : 0;
+    const int lane = (int)(threadIdx.x & (P - 1));
     const int ib = bra_of(ws.offs, ws.cbra, min(t, ws.total - 1));
     if (t >= ws.total) return;
     const int ik = ws.k0 + (int)(t - ws.offs[ib]);
@@ -323,41 +330,37 @@ __global__ void __launch_bounds__(128) eri_jk_kernel(JKArgs args) {
     load_xyz(args.bs, C, g.C);
     load_xyz(args.bs, D, g.D);
     T V[NA * NB * NC * ND];
-    if constexpr (!SPLIT) {
-        eri_block<LA, LB, LC, LD, true, T>(args.pp, args.bra.poff[ib], args.bra.np[ib], args.ket.poff[ik], args.ket.np[ik], g, V);
+#pragma unroll
+    for (int i = 0; i < NA * NB * NC * ND; ++i) V[i] = T(0);
+    const int pb0 = args.bra.poff[ib], pk0 = args.ket.poff[ik], npk = args.ket.np[ik];
+    const int nprim = args.bra.np[ib] * npk;
+    // primitive quartet idx = jb npk + jk, stepped by P without a division per step
+    int jb = lane / npk, jk = lane - jb * npk;
+    if constexpr (std::is_same<T, float>::value) {
+        const QuartetGeom32 g32 = geom32(g);
+        for (int idx = lane; idx < nprim; idx += P, jk += P) {
+            while (jk >= npk) { jk -= npk; ++jb; }
+            const PairRec32 Bp = load_rec32(args.pp.rec32, pb0 + jb), Kp = load_rec32(args.pp.rec32, pk0 + jk);
+            if (Bp.arg + Kp.arg > (float)PDG_PRIMITIVE_CUT) continue;
+            eri_prim32<LA, LB, LC, LD>(Bp, Kp, g32, V);
+        }
     } else {
-#pragma unroll
-        for (int i = 0; i < NA * NB * NC * ND; ++i) V[i] = T(0);
-        const int pb0 = args.bra.poff[ib], pk0 = args.ket.poff[ik], npk = args.ket.np[ik];
-        const int nprim = args.bra.np[ib] * npk;
-        // primitive quartet idx = jb npk + jk, stepped by P without a division per step
-        int jb = lane / npk, jk = lane - jb * npk;
-        if constexpr (std::is_same<T, float>::value) {
-            const QuartetGeom32 g32 = geom32(g);
-            for (int idx = lane; idx < nprim; idx += P, jk += P) {
-                while (jk >= npk) { jk -= npk; ++jb; }
-                const PairRec32 Bp = load_rec32(args.pp.rec32, pb0 + jb), Kp = load_rec32(args.pp.rec32, pk0 + jk);
-                if (Bp.arg + Kp.arg > (float)PDG_PRIMITIVE_CUT) continue;
-                eri_prim32<LA, LB, LC, LD>(Bp, Kp, g32, V);
-            }
-        } else {
-            for (int idx = lane; idx < nprim; idx += P, jk += P) {
-                while (jk >= npk) { jk -= npk; ++jb; }
-                const int xb = pb0 + jb, xk = pk0 + jk;
-                if (load_arg(args.pp.rec, xb) + load_arg(args.pp.rec, xk) > PDG_PRIMITIVE_CUT) continue;
-                eri_prim<LA, LB, LC, LD, T>(load_rec(args.pp.rec, xb), load_rec(args.pp.rec, xk), g, V);
-            }
+        for (int idx = lane; idx < nprim; idx += P, jk += P) {
+            while (jk >= npk) { jk -= npk; ++jb; }
+            const int xb = pb0 + jb, xk = pk0 + jk;
+            if (load_arg(args.pp.rec, xb) + load_arg(args.pp.rec, xk) > PDG_PRIMITIVE_CUT) continue;
+            eri_prim<LA, LB, LC, LD, T>(load_rec(args.pp.rec, xb), load_rec(args.pp.rec, xk), g, V);
         }
-        const unsigned mask = lane_group_mask(P);
-        for (int o = P >> 1; o > 0; o >>= 1) {
-#pragma unroll
-            for (int i = 0; i < NA * NB * NC * ND; ++i) V[i] += __shfl_xor_sync(mask, V[i], o);
-        }
-        // every lane of the group now holds the contracted block; up to three of them share the
-        // digest (J; K rows of a; K rows of b)
-        if (lane >= (P < 3 ? P : 3)) return;
     }
-    const int roles = SPLIT ? (P < 3 ? P : 3) : 1;
+    const unsigned mask = lane_group_mask(P);
+    for (int o = P >> 1; o > 0; o >>= 1) {
+#pragma unroll
+        for (int i = 0; i < NA * NB * NC * ND; ++i) V[i] += __shfl_xor_sync(mask, V[i], o);
+    }
+    // every lane of the group now holds the contracted block; up to three of them share the
+    // digest (J; K rows of a; K rows of b)
+    if (lane >= (P < 3 ? P : 3)) return;
+    const int roles = P < 3 ? P : 3;
     const bool do_j = lane == 0;
     const bool do_ka = roles == 3 ? lane == 1 : lane == 0;
     const bool do_kb = lane == roles - 1;
@@ -946,12 +949,22 @@ void launch_jk_p(JKArgs a, const QuartetBlock &b, bool doJ, bool doK, cudaStream
             else { eri_jk_warp_kernel<LA, LB, LC, LD, false, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
             return;
         }
-        constexpr bool SP = jk_split(LA, LB, LC, LD);
-        const int v = a.variant >= 0 ? a.variant : pdg_jk_variant[CB][CK].load(std::memory_order_relaxed);
-        const long long blocks = pdg_fill_work(a.work, b, SP ? kSplitLanesV[v] : kOneLane);
-        if (doJ && doK) { eri_jk_kernel<LA, LB, LC, LD, true, true, T, SP><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
-        else if (doJ) { eri_jk_kernel<LA, LB, LC, LD, true, false, T, SP><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
-        else { eri_jk_kernel<LA, LB, LC, LD, false, true, T, SP><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+        long long blocks;
+        if constexpr (jk_split(LA, LB, LC, LD)) {
+            int v = a.variant;
+            if (v < 0) {
+                v = pdg_jk_variant[CB][CK].load(std::memory_order_relaxed);
+                while (v + 1 < kNLanesV && pdg_work_threads(b, kSplitLanesV[v + 1]) <= kLaneThreads) ++v;
+            }
+            blocks = pdg_fill_work(a.work, b, kSplitLanesV[v]);
+        } else {
+            int v = 0;
+            while (v + 1 < kNWide && pdg_work_threads(b, kWideLanes[v + 1]) <= kLaneThreads / 2) ++v;
+            blocks = pdg_fill_work(a.work, b, kWideLanes[v]);
+        }
+        if (doJ && doK) { eri_jk_kernel<LA, LB, LC, LD, true, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+        else if (doJ) { eri_jk_kernel<LA, LB, LC, LD, true, false, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
+        else { eri_jk_kernel<LA, LB, LC, LD, false, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
     }
 }
 
