@@ -8,7 +8,7 @@
 //
 #include <algorithm>
 #include <cmath>
-#include <numeric>
+#include <cstring>
 #include <string>
 #include <atomic>
 #include <type_traits>
@@ -19,13 +19,19 @@ std::atomic<int> pdg_jk_variant[PDG_NPAIRCLASS][PDG_NPAIRCLASS];
 
 namespace {
 
-// Schwarz bound per shell pair: Q = sqrt(max_ab |(ab|ab)|) with the true normalisation.
+// Schwarz bound per shell pair: Q = sqrt(max_ab |(ab|ab)|) with the true normalisation, eight lanes to a
+// pair (one for d with d: one primitive pair).  Without the primitive-quartet cut, because a primitive pair
+// cut in (ab|ab) can still contribute to (ab|cd) against a compact ket pair.  In one lane the 1296
+// primitive quartets of two sixfold contracted s shells took 0.25 ms of every new geometry.
+__host__ __device__ constexpr int schwarz_lanes(int la, int lb) { return la + lb < 4 ? 8 : 1; }
+
 template <int LA, int LB>
 __global__ void __launch_bounds__(64) schwarz_kernel(const int n, const int *__restrict__ shA,
                                                      const int *__restrict__ shB, const int *__restrict__ poff,
                                                      const int *__restrict__ np, PrimPairs pp, DeviceBasis bs,
                                                      double *__restrict__ Q) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int P = schwarz_lanes(LA, LB);
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) / P, lane = threadIdx.x & (P - 1);
     if (t >= n) return;
     constexpr int NA = ncart(LA), NB = ncart(LB);
     QuartetGeom g;
@@ -34,16 +40,24 @@ __global__ void __launch_bounds__(64) schwarz_kernel(const int n, const int *__r
 #pragma unroll
     for (int c = 0; c < 3; ++c) { g.C[c] = g.A[c]; g.D[c] = g.B[c]; }
     double V[NA * NB * NA * NB];
-    eri_block<LA, LB, LA, LB, false>(pp, poff[t], np[t], poff[t], np[t], g, V);
+#pragma unroll
+    for (int i = 0; i < NA * NB * NA * NB; ++i) V[i] = 0.0;
+    const int p0 = poff[t], npr = np[t];
+    for (int k = lane; k < npr * npr; k += P)
+        eri_prim<LA, LB, LA, LB>(load_rec(pp.rec, p0 + k / npr), load_rec(pp.rec, p0 + k % npr), g, V);
+    const unsigned mask = lane_group_mask(P);
     double m = 0.0;
 #pragma unroll
     for (int a = 0; a < NA; ++a)
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
+            double v = V[((a * NB + b) * NA + a) * NB + b];
+#pragma unroll
+            for (int o = P >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
             const double nn = comp_norm(LA, a) * comp_norm(LB, b);
-            m = fmax(m, fabs(V[((a * NB + b) * NA + a) * NB + b]) * nn * nn);
+            m = fmax(m, fabs(v) * nn * nn);
         }
-    Q[t] = sqrt(m);
+    if (lane == 0) Q[t] = sqrt(m);
 }
 
 struct VariantInit {
@@ -63,25 +77,39 @@ template <int C>
 void launch_schwarz_t(int n, const int *shA, const int *shB, const int *poff, const int *np, const PrimPairs &pp,
                       const DeviceBasis &bs, double *Q, cudaStream_t st) {
     if (n == 0) return;
-    { schwarz_kernel<PLA[C], PLB[C]><<<(n + 63) / 64, 64, 0, st>>>(n, shA, shB, poff, np, pp, bs, Q); pdg_count_launch(); }
+    { schwarz_kernel<PLA[C], PLB[C]><<<(n * schwarz_lanes(PLA[C], PLB[C]) + 63) / 64, 64, 0, st>>>(n, shA, shB, poff, np, pp, bs, Q); pdg_count_launch(); }
 }
 typedef void (*schwarz_launcher)(int, const int *, const int *, const int *, const int *, const PrimPairs &,
                                  const DeviceBasis &, double *, cudaStream_t);
 const schwarz_launcher schwarz_table[PDG_NPAIRCLASS] = {launch_schwarz_t<0>, launch_schwarz_t<1>, launch_schwarz_t<2>,
                                                         launch_schwarz_t<3>, launch_schwarz_t<4>, launch_schwarz_t<5>};
 
-// Upload into the context's named buffer pool (grown when needed, never freed before the context
-// is destroyed), stream-ordered on the context's non-blocking stream and complete on return, so a
-// new geometry reuses the device memory of the last one without allocating.
-template <typename T>
-int upload(pdg_context *ctx, const std::string &name, T **dst, const std::vector<T> &src) {
-    *dst = (T *)pdg_pool(ctx, name.c_str(), std::max<size_t>(1, src.size()) * sizeof(T));
-    if (!*dst) { pdg_set_error("device buffer allocation failed (%s)", name.c_str()); return PDG_ERR_ALLOC; }
-    if (src.empty()) return PDG_OK;
-    PDG_CUDA(cudaMemcpyAsync(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
-    PDG_CUDA(cudaStreamSynchronize(ctx->stream));
-    return PDG_OK;
-}
+// Host arrays gathered for one transfer into one pool buffer: add() gives an array's place, send() copies all
+// (stream-ordered on the context's non-blocking stream and complete on return).  The pool's buffer grows when
+// needed and stays, so that a new geometry reuses the last one's.  A copy and its wait take some 10 us
+// each, and the lists of a geometry are some 80 arrays.
+class Staged {
+    std::vector<char> bytes;
+
+public:
+    template <typename T>
+    size_t add(const T *src, size_t n) {
+        const size_t at = (bytes.size() + 15) / 16 * 16;
+        bytes.resize(at + n * sizeof(T));
+        if (n) std::memcpy(bytes.data() + at, src, n * sizeof(T));
+        return at;
+    }
+    template <typename T>
+    size_t add(const std::vector<T> &v) { return add(v.data(), v.size()); }
+    int send(pdg_context *ctx, const char *name, char **dst) {
+        *dst = (char *)pdg_pool(ctx, name, std::max<size_t>(16, bytes.size()));
+        if (!*dst) { pdg_set_error("device buffer allocation failed (%s)", name); return PDG_ERR_ALLOC; }
+        if (bytes.empty()) return PDG_OK;
+        PDG_CUDA(cudaMemcpyAsync(*dst, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, ctx->stream));
+        PDG_CUDA(cudaStreamSynchronize(ctx->stream));
+        return PDG_OK;
+    }
+};
 
 std::string cname(const char *base, int c) { return std::string(base) + "." + std::to_string(c); }
 
@@ -110,15 +138,60 @@ void pdg_free_pairs(pdg_context *ctx) {
     ctx->blocks_thr = -1.0;
 }
 
-// Build primitive-pair data and Schwarz-sorted shell-pair lists for the current geometry.
+// Exponent argument of a primitive pair, without fused operations: host and device count the same pairs.
+__host__ __device__ __forceinline__ double primitive_arg(double ea, double eb, double r2) {
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(__ddiv_rn(__dmul_rn(ea, eb), __dadd_rn(ea, eb)), r2);
+#else
+    return ea * eb / (ea + eb) * r2;
+#endif
+}
+
+// The primitive pairs of each shell pair (A, B, first primitive pair, squared distance), in the order the host
+// counted them: one thread per shell pair.
+__global__ void __launch_bounds__(128) pair_fill_kernel(int n, const int *__restrict__ shA, const int *__restrict__ shB,
+                                                        const int *__restrict__ off, const double *__restrict__ dist2,
+                                                        DeviceBasis bs, PrimPairs pp, double2 *__restrict__ rec,
+                                                        float4 *__restrict__ rec32) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int A = shA[t], B = shB[t];
+    double rA[3], rB[3];
+    load_xyz(bs, A, rA);
+    load_xyz(bs, B, rB);
+    const double r2 = dist2[t];
+    int i = off[t];
+    for (int pa = bs.sh_poff[A]; pa < bs.sh_poff[A] + bs.sh_np[A]; ++pa) {
+        const double ea = bs.prim_exp[pa], ca = bs.prim_coef[pa];
+        for (int pb = bs.sh_poff[B]; pb < bs.sh_poff[B] + bs.sh_np[B]; ++pb) {
+            const double eb = bs.prim_exp[pb], p = ea + eb, arg = primitive_arg(ea, eb, r2);
+            if (arg > PDG_PRIMITIVE_CUT) continue;
+            const double x = (ea * rA[0] + eb * rB[0]) / p, y = (ea * rA[1] + eb * rB[1]) / p, z = (ea * rA[2] + eb * rB[2]) / p;
+            const double K = exp(-arg) * ca * bs.prim_coef[pb], Kp = K / p, hp = 0.5 / p;
+            pp.a[i] = ea; pp.b[i] = eb;
+            pp.Px[i] = x; pp.Py[i] = y; pp.Pz[i] = z;
+            pp.K[i] = K; pp.arg[i] = arg; pp.Kp[i] = Kp; pp.hp[i] = hp;
+            rec[4 * i] = make_double2(p, x); rec[4 * i + 1] = make_double2(y, z);
+            rec[4 * i + 2] = make_double2(Kp, hp); rec[4 * i + 3] = make_double2(arg, ea);
+            rec32[2 * i] = make_float4((float)p, (float)(x - rA[0]), (float)(y - rA[1]), (float)(z - rA[2]));
+            rec32[2 * i + 1] = make_float4((float)Kp, (float)hp, (float)arg, 0.0f);
+            ++i;
+        }
+    }
+}
+
+// Build primitive-pair data and Schwarz-sorted shell-pair lists for the current geometry.  The host counts
+// the primitive pairs of each shell pair and sorts; the device forms them and the bounds, between two
+// transfers up and one down (formed on the host and sent array by array, each waited for: 8 ms of a new
+// geometry of 32 waters, 1.6 ms of one of 4).
 int pdg_ensure_pairs(pdg_context *ctx) {
     if (ctx->pairs[0].shA || ctx->pp.a) return PDG_OK;
     ProfScope prof(ctx, "pairs");
     const auto &sh = ctx->shells;
     const int ns = (int)sh.size();
     std::vector<int> cshA[PDG_NPAIRCLASS], cshB[PDG_NPAIRCLASS], cpoff[PDG_NPAIRCLASS], cnp[PDG_NPAIRCLASS];
-    std::vector<double> va, vb, vPx, vPy, vPz, vK, varg, vKp, vhp;
-    std::vector<int> pair_atomA;   // atom of the first centre of each primitive pair
+    std::vector<double> cr2[PDG_NPAIRCLASS];
+    int npp = 0;
     for (int i = 0; i < ns; ++i) {
         for (int j = 0; j <= i; ++j) {
             int A = i, B = j;
@@ -126,112 +199,99 @@ int pdg_ensure_pairs(pdg_context *ctx) {
             const double *rA = &ctx->xyz[3 * sh[A].atom], *rB = &ctx->xyz[3 * sh[B].atom];
             const double dx = rA[0] - rB[0], dy = rA[1] - rB[1], dz = rA[2] - rB[2];
             const double r2 = dx * dx + dy * dy + dz * dz;
-            const int off = (int)va.size();
-            for (int pa = 0; pa < sh[A].np; ++pa) {
-                const double ea = ctx->prim_exp[sh[A].poff + pa], ca = ctx->prim_coef[sh[A].poff + pa];
-                for (int pb = 0; pb < sh[B].np; ++pb) {
-                    const double eb = ctx->prim_exp[sh[B].poff + pb], cb = ctx->prim_coef[sh[B].poff + pb];
-                    const double p = ea + eb;
-                    const double arg = ea * eb / p * r2;
-                    if (arg > PDG_PRIMITIVE_CUT) continue;
-                    va.push_back(ea);
-                    vb.push_back(eb);
-                    vPx.push_back((ea * rA[0] + eb * rB[0]) / p);
-                    vPy.push_back((ea * rA[1] + eb * rB[1]) / p);
-                    vPz.push_back((ea * rA[2] + eb * rB[2]) / p);
-                    vK.push_back(std::exp(-arg) * ca * cb);
-                    varg.push_back(arg);
-                    vKp.push_back(vK.back() / p);
-                    vhp.push_back(0.5 / p);
-                    pair_atomA.push_back(sh[A].atom);
-                }
-            }
-            const int cnt = (int)va.size() - off;
+            int cnt = 0;
+            for (int pa = 0; pa < sh[A].np; ++pa)
+                for (int pb = 0; pb < sh[B].np; ++pb)
+                    cnt += !(primitive_arg(ctx->prim_exp[sh[A].poff + pa], ctx->prim_exp[sh[B].poff + pb], r2) > PDG_PRIMITIVE_CUT);
             if (cnt == 0) continue;
             const int c = pair_class(sh[A].l, sh[B].l);
             cshA[c].push_back(A);
             cshB[c].push_back(B);
-            cpoff[c].push_back(off);
+            cpoff[c].push_back(npp);
             cnp[c].push_back(cnt);
+            cr2[c].push_back(r2);
+            npp += cnt;
         }
     }
-    ctx->npp = (int)va.size();
-    PDG_CHECK(upload(ctx, "pp.a", &ctx->pp.a, va));
-    PDG_CHECK(upload(ctx, "pp.b", &ctx->pp.b, vb));
-    PDG_CHECK(upload(ctx, "pp.Px", &ctx->pp.Px, vPx));
-    PDG_CHECK(upload(ctx, "pp.Py", &ctx->pp.Py, vPy));
-    PDG_CHECK(upload(ctx, "pp.Pz", &ctx->pp.Pz, vPz));
-    PDG_CHECK(upload(ctx, "pp.K", &ctx->pp.K, vK));
-    PDG_CHECK(upload(ctx, "pp.arg", &ctx->pp.arg, varg));
-    PDG_CHECK(upload(ctx, "pp.Kp", &ctx->pp.Kp, vKp));
-    PDG_CHECK(upload(ctx, "pp.hp", &ctx->pp.hp, vhp));
+    ctx->npp = npp;
+    ctx->hostArg.clear();
     {
-        std::vector<double> rec(8 * va.size());
-        for (size_t i = 0; i < va.size(); ++i) {
-            double *r = &rec[8 * i];
-            r[0] = va[i] + vb[i]; r[1] = vPx[i]; r[2] = vPy[i]; r[3] = vPz[i];
-            r[4] = vKp[i]; r[5] = vhp[i]; r[6] = varg[i]; r[7] = va[i];
+        const size_t n = std::max(1, npp);
+        double *soa = (double *)pdg_pool(ctx, "pp.soa", 9 * n * sizeof(double));
+        double2 *rec = (double2 *)pdg_pool(ctx, "pp.rec", 4 * n * sizeof(double2));
+        float4 *rec32 = (float4 *)pdg_pool(ctx, "pp.rec32", 2 * n * sizeof(float4));
+        if (!soa || !rec || !rec32) { pdg_set_error("device buffer allocation failed (primitive pairs)"); return PDG_ERR_ALLOC; }
+        // the unsorted lists, all classes behind one another
+        std::vector<int> A, B, O, N;
+        std::vector<double> R;
+        size_t first[PDG_NPAIRCLASS + 1] = {0};
+        for (int c = 0; c < PDG_NPAIRCLASS; ++c) {
+            A.insert(A.end(), cshA[c].begin(), cshA[c].end());
+            B.insert(B.end(), cshB[c].begin(), cshB[c].end());
+            O.insert(O.end(), cpoff[c].begin(), cpoff[c].end());
+            N.insert(N.end(), cnp[c].begin(), cnp[c].end());
+            R.insert(R.end(), cr2[c].begin(), cr2[c].end());
+            first[c + 1] = A.size();
         }
-        double *drec = nullptr;
-        PDG_CHECK(upload(ctx, "pp.rec", &drec, rec));
-        ctx->pp.rec = reinterpret_cast<const double2 *>(drec);
-        std::vector<float> rec32(8 * va.size());
-        for (size_t i = 0; i < va.size(); ++i) {
-            float *r = &rec32[8 * i];
-            const double *rA = &ctx->xyz[3 * pair_atomA[i]];
-            r[0] = (float)(va[i] + vb[i]);
-            r[1] = (float)(vPx[i] - rA[0]); r[2] = (float)(vPy[i] - rA[1]); r[3] = (float)(vPz[i] - rA[2]);
-            r[4] = (float)vKp[i]; r[5] = (float)vhp[i]; r[6] = (float)varg[i]; r[7] = 0.0f;
+        const int np = (int)A.size();
+        Staged up;
+        const size_t oA = up.add(A), oB = up.add(B), oO = up.add(O), oN = up.add(N), oR = up.add(R);
+        char *d = nullptr;
+        PDG_CHECK(up.send(ctx, "pairs.unsorted", &d));
+        const int *dA = (const int *)(d + oA), *dB = (const int *)(d + oB), *dO = (const int *)(d + oO), *dN = (const int *)(d + oN);
+        double *dQ = (double *)pdg_pool(ctx, "schwarz.Q", std::max(1, np) * sizeof(double));
+        if (!dQ) { pdg_set_error("device buffer allocation failed (schwarz.Q)"); return PDG_ERR_ALLOC; }
+        PrimPairs pp;
+        double **arrays[] = {&pp.a, &pp.b, &pp.Px, &pp.Py, &pp.Pz, &pp.K, &pp.arg, &pp.Kp, &pp.hp};
+        for (int k = 0; k < 9; ++k) *arrays[k] = soa + k * n;
+        pp.rec = rec;
+        pp.rec32 = rec32;
+        std::vector<double> allQ(np);
+        if (np > 0) {
+            { pair_fill_kernel<<<(np + 127) / 128, 128, 0, ctx->stream>>>(np, dA, dB, dO, (const double *)(d + oR), ctx->dbasis, pp, rec, rec32); pdg_count_launch(); }
+            {
+                ClassFork fork(ctx);
+                for (int c = 0; c < PDG_NPAIRCLASS; ++c)
+                    schwarz_table[c]((int)(first[c + 1] - first[c]), dA + first[c], dB + first[c], dO + first[c], dN + first[c], pp,
+                                     ctx->dbasis, dQ + first[c], fork.stream(1.0));
+            }
+            PDG_CUDA(cudaGetLastError());
+            PDG_CUDA(cudaMemcpyAsync(allQ.data(), dQ, np * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+            PDG_CUDA(cudaStreamSynchronize(ctx->stream));
         }
-        float *drec32 = nullptr;
-        PDG_CHECK(upload(ctx, "pp.rec32", &drec32, rec32));
-        ctx->pp.rec32 = reinterpret_cast<const float4 *>(drec32);
+        ctx->pp = pp;
+        for (int c = 0; c < PDG_NPAIRCLASS; ++c) ctx->hostQ[c].assign(allQ.begin() + first[c], allQ.begin() + first[c + 1]);
     }
-    ctx->hostArg = varg;
-    // Schwarz bounds on the unsorted lists, then sort each class by Q descending.
+    // each class by primitive-count bucket, then by Schwarz bound (descending) inside a bucket
+    Staged up;
+    size_t at[PDG_NPAIRCLASS][6] = {};
+    int ngroup[PDG_NPAIRCLASS] = {}, slots[PDG_NPAIRCLASS] = {};
+    struct Key {
+        double Q;
+        int bucket, index;
+    };
+    std::vector<Key> key;
     for (int c = 0; c < PDG_NPAIRCLASS; ++c) {
         const int n = (int)cshA[c].size();
-        ctx->hostQ[c].clear();
         ctx->bucket_start[c].assign(PDG_NBUCKET + 1, 0);
         ctx->qmax[c] = 0.0;
+        ctx->hostPoff[c].resize(n);
+        ctx->hostNp[c].resize(n);
         if (n == 0) continue;
-        int *dA = nullptr, *dB = nullptr, *dO = nullptr, *dN = nullptr;
-        double *dQ = nullptr;
-        PDG_CHECK(upload(ctx, "schwarz.A", &dA, cshA[c]));
-        PDG_CHECK(upload(ctx, "schwarz.B", &dB, cshB[c]));
-        PDG_CHECK(upload(ctx, "schwarz.O", &dO, cpoff[c]));
-        PDG_CHECK(upload(ctx, "schwarz.N", &dN, cnp[c]));
-        dQ = (double *)pdg_pool(ctx, "schwarz.Q", n * sizeof(double));
-        if (!dQ) { pdg_set_error("device buffer allocation failed (schwarz.Q)"); return PDG_ERR_ALLOC; }
-        schwarz_table[c](n, dA, dB, dO, dN, ctx->pp, ctx->dbasis, dQ, ctx->stream);
-        PDG_CUDA(cudaGetLastError());
-        std::vector<double> Q(n);
-        PDG_CUDA(cudaMemcpyAsync(Q.data(), dQ, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        PDG_CUDA(cudaStreamSynchronize(ctx->stream));
-        // by primitive-count bucket, then by Schwarz bound (descending) inside a bucket
-        std::vector<int> order(n);
-        std::iota(order.begin(), order.end(), 0);
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-            const int bx = np_bucket(cnp[c][x]), by = np_bucket(cnp[c][y]);
-            return bx != by ? bx < by : Q[x] > Q[y];
+        key.resize(n);
+        for (int k = 0; k < n; ++k) key[k] = Key{ctx->hostQ[c][k] == ctx->hostQ[c][k] ? ctx->hostQ[c][k] : 0.0, np_bucket(cnp[c][k]), k};
+        std::sort(key.begin(), key.end(), [](const Key &x, const Key &y) {
+            return x.bucket != y.bucket ? x.bucket < y.bucket : x.Q != y.Q ? x.Q > y.Q : x.index < y.index;
         });
-        std::vector<int> sA(n), sB(n), sO(n), sN(n);
-        std::vector<double> sQ(n);
+        std::vector<int> sA(n), sB(n);
+        auto &sO = ctx->hostPoff[c], &sN = ctx->hostNp[c];
+        auto &sQ = ctx->hostQ[c];
         for (int k = 0; k < n; ++k) {
-            sA[k] = cshA[c][order[k]]; sB[k] = cshB[c][order[k]];
-            sO[k] = cpoff[c][order[k]]; sN[k] = cnp[c][order[k]];
-            sQ[k] = Q[order[k]];
+            const int o = key[k].index;
+            sA[k] = cshA[c][o]; sB[k] = cshB[c][o];
+            sO[k] = cpoff[c][o]; sN[k] = cnp[c][o];
+            sQ[k] = key[k].Q;
         }
-        PairList &pl = ctx->pairs[c];
-        pl.n = n;
-        PDG_CHECK(upload(ctx, cname("pairs.shA", c), &pl.shA, sA));
-        PDG_CHECK(upload(ctx, cname("pairs.shB", c), &pl.shB, sB));
-        PDG_CHECK(upload(ctx, cname("pairs.poff", c), &pl.poff, sO));
-        PDG_CHECK(upload(ctx, cname("pairs.np", c), &pl.np, sN));
-        PDG_CHECK(upload(ctx, cname("pairs.Q", c), &pl.Q, sQ));
-        ctx->hostQ[c] = sQ;
-        ctx->hostPoff[c] = sO;
-        ctx->hostNp[c] = sN;
         ctx->qmax[c] = *std::max_element(sQ.begin(), sQ.end());
         auto &bs = ctx->bucket_start[c];
         bs.assign(PDG_NBUCKET + 1, n);
@@ -242,25 +302,38 @@ int pdg_ensure_pairs(pdg_context *ctx) {
         std::vector<int> goff, gfirst;  // first slot; first pair and pair count, by group
         auto &bg = ctx->bucket_group[c];
         bg.assign(PDG_NBUCKET, 0);
-        int slots = 0;
         for (int kb = 0; kb < PDG_NBUCKET; ++kb) {
             bg[kb] = (int)goff.size();
             for (int k = bs[kb]; k < bs[kb + 1]; k += 32) {
                 const int e = std::min(k + 32, bs[kb + 1]);
-                goff.push_back(slots);
+                goff.push_back(slots[c]);
                 gfirst.push_back(k);
                 gfirst.push_back(e - k);
-                slots += *std::max_element(sN.begin() + k, sN.begin() + e);
+                slots[c] += *std::max_element(sN.begin() + k, sN.begin() + e);
             }
         }
-        const int ng = (int)goff.size();
-        if (ng & 1) goff.push_back(0);  // the (first, count) pairs behind start on 8 bytes
+        ngroup[c] = (int)goff.size();
+        if (ngroup[c] & 1) goff.push_back(0);  // the (first, count) pairs behind start on 8 bytes
         goff.insert(goff.end(), gfirst.begin(), gfirst.end());
-        int *dg = nullptr;
-        PDG_CHECK(upload(ctx, cname("pairs.goff", c), &dg, goff));
-        double2 *grec = (double2 *)pdg_pool(ctx, cname("pairs.grec", c).c_str(), (size_t)slots * 128 * sizeof(double2));
-        float4 *grec32 = (float4 *)pdg_pool(ctx, cname("pairs.grec32", c).c_str(), (size_t)slots * 64 * sizeof(float4));
+        at[c][0] = up.add(sA); at[c][1] = up.add(sB); at[c][2] = up.add(sO);
+        at[c][3] = up.add(sN); at[c][4] = up.add(sQ); at[c][5] = up.add(goff);
+    }
+    char *d = nullptr;
+    PDG_CHECK(up.send(ctx, "pairs.lists", &d));
+    for (int c = 0; c < PDG_NPAIRCLASS; ++c) {
+        PairList &pl = ctx->pairs[c];
+        pl.n = (int)cshA[c].size();
+        if (pl.n == 0) continue;
+        pl.shA = (int *)(d + at[c][0]);
+        pl.shB = (int *)(d + at[c][1]);
+        pl.poff = (int *)(d + at[c][2]);
+        pl.np = (int *)(d + at[c][3]);
+        pl.Q = (double *)(d + at[c][4]);
+        const int *dg = (const int *)(d + at[c][5]);
+        double2 *grec = (double2 *)pdg_pool(ctx, cname("pairs.grec", c).c_str(), (size_t)slots[c] * 128 * sizeof(double2));
+        float4 *grec32 = (float4 *)pdg_pool(ctx, cname("pairs.grec32", c).c_str(), (size_t)slots[c] * 64 * sizeof(float4));
         if (!grec || !grec32) { pdg_set_error("device buffer allocation failed (pairs.grec)"); return PDG_ERR_ALLOC; }
+        const int ng = ngroup[c];
         { ket_group_kernel<<<(ng + 3) / 4, 128, 0, ctx->stream>>>(ng, dg, reinterpret_cast<const int2 *>(dg + ng + (ng & 1)), pl, ctx->pp, grec, grec32); pdg_count_launch(); }
         PDG_CUDA(cudaGetLastError());
         pl.grec = grec;
@@ -270,18 +343,95 @@ int pdg_ensure_pairs(pdg_context *ctx) {
     return PDG_OK;
 }
 
-// cbra[k] = bra pair of quartet min(4k, total - 1) (binary search of the prefix sums).
-__global__ void bra_map_kernel(const long long *__restrict__ offs, int nbra, long long total, long long nk,
-                               int *__restrict__ cbra) {
-    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (k >= nk) return;
-    const long long t = min(4 * k, total - 1);
-    int lo = 0, hi = nbra;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (offs[mid] <= t) lo = mid; else hi = mid;
+// One (bra class, ket class, ket bucket) of the work list while it is built.
+struct BlockDesc {
+    const double *need, *Qk;      // what a bra pair needs of a ket (threshold / its bound); bounds of the ket class
+    const int *np;                // primitive pairs of the bra pairs
+    int nb, k0, nk, same;
+    long long *offs, *woffs;      // prefix sums over the bras (nb + 1 each)
+    long long total, wtotal;      // quartets and (bra, ket group) items
+    int *cbra, *wbra;             // their bra maps (bra_of)
+};
+
+// Prefix sums over the bra pairs of a bucket's surviving kets (pdg_ket_count) and of their groups of 32, with
+// the totals and the bras' primitive pairs summed over the quartets: one CTA per descriptor.
+__global__ void __launch_bounds__(1024) block_offsets_kernel(const BlockDesc *__restrict__ desc, long long *__restrict__ totals) {
+    const BlockDesc b = desc[blockIdx.x];
+    __shared__ long long ws[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    long long base = 0, wbase = 0, prims = 0;
+    if (threadIdx.x == 0) b.offs[0] = b.woffs[0] = 0;
+    for (int i0 = 0; i0 < b.nb; i0 += 1024) {
+        const int i = i0 + threadIdx.x;
+        long long cnt = 0;
+        if (i < b.nb) {  // the bucket is sorted by Q descending: the kets with Q >= need are a prefix
+            const double need = b.need[i];
+            int lo = 0, hi = b.nk;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (b.Qk[b.k0 + mid] >= need) lo = mid + 1; else hi = mid;
+            }
+            cnt = lo;
+            if (b.same) cnt = min(cnt, (long long)max(0, i - b.k0 + 1));
+            prims += cnt * b.np[i];
+        }
+        long long s = cnt, g = (cnt + 31) / 32;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, s, o), v = __shfl_up_sync(0xffffffffu, g, o);
+            if (lane >= o) { s += u; g += v; }
+        }
+        if (lane == 31) { ws[0][w] = s; ws[1][w] = g; }
+        __syncthreads();
+        if (w == 0) {
+            long long x = ws[0][lane], y = ws[1][lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long u = __shfl_up_sync(0xffffffffu, x, o), v = __shfl_up_sync(0xffffffffu, y, o);
+                if (lane >= o) { x += u; y += v; }
+            }
+            ws[0][lane] = x;
+            ws[1][lane] = y;
+        }
+        __syncthreads();
+        if (i < b.nb) {
+            b.offs[i + 1] = base + s + (w ? ws[0][w - 1] : 0);
+            b.woffs[i + 1] = wbase + g + (w ? ws[1][w - 1] : 0);
+        }
+        base += ws[0][31];
+        wbase += ws[1][31];
+        __syncthreads();
     }
-    cbra[k] = lo;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) prims += __shfl_xor_sync(0xffffffffu, prims, o);
+    if (lane == 0) ws[0][w] = prims;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        prims = 0;
+        for (int k = 0; k < 32; ++k) prims += ws[0][k];
+        totals[3 * blockIdx.x] = base;
+        totals[3 * blockIdx.x + 1] = wbase;
+        totals[3 * blockIdx.x + 2] = prims;
+    }
+}
+
+// The bra maps: entry k = bra pair of item min(4k, total - 1) (binary search of the prefix sums), of the
+// quartets (blockIdx.z 0) and of the (bra, ket group) items (1) of descriptor blockIdx.y.
+__global__ void __launch_bounds__(256) bra_map_kernel(const BlockDesc *__restrict__ desc) {
+    const BlockDesc b = desc[blockIdx.y];
+    const long long *__restrict__ offs = blockIdx.z ? b.woffs : b.offs;
+    const long long total = blockIdx.z ? b.wtotal : b.total;
+    int *__restrict__ map = blockIdx.z ? b.wbra : b.cbra;
+    const long long n = (total - 1) / 4 + 2;
+    for (long long k = blockIdx.x * 256LL + threadIdx.x; k < n; k += gridDim.x * 256LL) {
+        const long long t = min(4 * k, total - 1);
+        int lo = 0, hi = b.nb;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (offs[mid] <= t) lo = mid; else hi = mid;
+        }
+        map[k] = lo;
+    }
 }
 
 long long pdg_ket_count(const pdg_context *ctx, int cb, int ck, int ib, int k0, int nk, double thr) {
@@ -299,57 +449,112 @@ long long pdg_ket_count(const pdg_context *ctx, int cb, int ck, int ib, int k0, 
 // Screened work list: for each (bra class >= ket class) block and each primitive-count bucket of the
 // ket class, prefix sums over bra pairs of the number of ket pairs of the bucket with
 // Q_bra * Q_ket >= thr; inside one class a quartet is counted once, with its ket at or before its bra
-// in the class order.
+// in the class order (pdg_ket_count is the rule).
 int pdg_build_blocks(pdg_context *ctx, double thr) {
     if (ctx->blocks_thr == thr && !ctx->blocks.empty()) return PDG_OK;
     ctx->blocks.clear();
-    int nbuf = 0;
+    // what a bra needs of a ket, thr / Q_bra (infinite without a bound), by class
+    Staged needs;
+    size_t need_at[PDG_NPAIRCLASS] = {};
+    std::vector<double> need;
+    for (int c = 0; c < PDG_NPAIRCLASS; ++c) {
+        need.resize(ctx->hostQ[c].size());
+        for (size_t i = 0; i < need.size(); ++i) need[i] = ctx->hostQ[c][i] > 0.0 ? thr / ctx->hostQ[c][i] : HUGE_VAL;
+        need_at[c] = needs.add(need);
+    }
+    struct Sub {
+        int cb, ck, kb;
+    };
+    std::vector<Sub> subs;
+    std::vector<BlockDesc> desc;
+    size_t noffs = 0;
     for (int cb = 0; cb < PDG_NPAIRCLASS; ++cb) {
-        const auto &Qb = ctx->hostQ[cb];
-        if (Qb.empty()) continue;
-        for (int ck = 0; ck <= cb; ++ck) {
-            if (ctx->hostQ[ck].empty()) continue;
-            QuartetBlock qb{};
-            qb.cb = cb;
-            qb.ck = ck;
-            const int lt = PLA[cb] + PLB[cb] + PLA[ck] + PLB[ck];
-            const double per = 20.0 + (lt / 2 + 1) * ncart(PLA[cb]) * ncart(PLB[cb]) * ncart(PLA[ck]) * ncart(PLB[ck]);
+        const int nb = (int)ctx->hostQ[cb].size();
+        if (nb == 0) continue;
+        for (int ck = 0; ck <= cb; ++ck)
             for (int kb = 0; kb < PDG_NBUCKET; ++kb) {
+                if (ctx->hostQ[ck].empty()) continue;
                 const int k0 = ctx->bucket_start[ck][kb], nk = ctx->bucket_start[ck][kb + 1] - k0;
                 if (nk <= 0) continue;
-                // quartets, and behind them the (bra, group of 32 kets) items, as prefix sums over the bras
-                const size_t nb = Qb.size();
-                std::vector<long long> offs(2 * (nb + 1), 0);
-                const double npk = ctx->hostNp[ck][k0];
-                long long *woffs = &offs[nb + 1];
-                for (size_t i = 0; i < nb; ++i) {
-                    const long long cnt = pdg_ket_count(ctx, cb, ck, (int)i, k0, nk, thr);
-                    offs[i + 1] = offs[i] + cnt;
-                    woffs[i + 1] = woffs[i] + (cnt + 31) / 32;
-                    qb.cost += per * npk * ctx->hostNp[cb][i] * cnt;
-                }
-                if (offs[nb] == 0) continue;
-                auto &sb = qb.sub[qb.nsub++];
-                sb.total = offs[nb];
-                sb.wtotal = woffs[nb];
-                sb.k0 = k0;
-                sb.nk = nk;
-                sb.bucket = kb;
-                sb.g0 = ctx->bucket_group[ck][kb];
-                PDG_CHECK(upload(ctx, cname("blocks.offs", nbuf), &sb.offs, offs));
-                sb.woffs = sb.offs + nb + 1;
-                const long long nmap = (sb.total - 1) / 4 + 2, wmap = (sb.wtotal - 1) / 4 + 2;
-                sb.cbra = (int *)pdg_pool(ctx, cname("blocks.cbra", nbuf).c_str(), (nmap + wmap) * sizeof(int));
-                if (!sb.cbra) { pdg_set_error("device buffer allocation failed (blocks.cbra)"); return PDG_ERR_ALLOC; }
-                sb.wbra = sb.cbra + nmap;
-                { bra_map_kernel<<<(unsigned)((nmap + 255) / 256), 256, 0, ctx->stream>>>(sb.offs, (int)nb, sb.total, nmap, sb.cbra); pdg_count_launch(); }
-                { bra_map_kernel<<<(unsigned)((wmap + 255) / 256), 256, 0, ctx->stream>>>(sb.woffs, (int)nb, sb.wtotal, wmap, sb.wbra); pdg_count_launch(); }
-                PDG_CUDA(cudaGetLastError());
-                qb.total += sb.total;
-                ++nbuf;
+                subs.push_back(Sub{cb, ck, kb});
+                desc.push_back(BlockDesc{nullptr, ctx->pairs[ck].Q, ctx->pairs[cb].np, nb, k0, nk, cb == ck, nullptr, nullptr, 0, 0, nullptr, nullptr});
+                noffs += 2 * ((size_t)nb + 1);
             }
-            if (qb.nsub > 0) ctx->blocks.push_back(qb);
+    }
+    const int nsub = (int)subs.size();
+    if (nsub == 0) { ctx->blocks_thr = thr; return PDG_OK; }
+    long long *offs = (long long *)pdg_pool(ctx, "blocks.offs", noffs * sizeof(long long));
+    long long *dtot = (long long *)pdg_pool(ctx, "blocks.totals", 3 * nsub * sizeof(long long));
+    if (!offs || !dtot) { pdg_set_error("device buffer allocation failed (blocks.offs)"); return PDG_ERR_ALLOC; }
+    char *dneed = nullptr, *ddesc = nullptr;
+    PDG_CHECK(needs.send(ctx, "blocks.need", &dneed));
+    for (int k = 0; k < nsub; ++k) {
+        desc[k].need = (const double *)(dneed + need_at[subs[k].cb]);
+        desc[k].offs = offs;
+        desc[k].woffs = offs + desc[k].nb + 1;
+        offs += 2 * ((size_t)desc[k].nb + 1);
+    }
+    {
+        Staged up;
+        up.add(desc);
+        PDG_CHECK(up.send(ctx, "blocks.desc", &ddesc));
+    }
+    { block_offsets_kernel<<<nsub, 1024, 0, ctx->stream>>>((const BlockDesc *)ddesc, dtot); pdg_count_launch(); }
+    PDG_CUDA(cudaGetLastError());
+    std::vector<long long> tot(3 * nsub);
+    PDG_CUDA(cudaMemcpyAsync(tot.data(), dtot, tot.size() * sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream));
+    PDG_CUDA(cudaStreamSynchronize(ctx->stream));
+    // the bra maps of the lists that hold quartets
+    std::vector<BlockDesc> live;
+    size_t nmap = 0;
+    long long longest = 0;
+    for (int k = 0; k < nsub; ++k) {
+        desc[k].total = tot[3 * k];
+        desc[k].wtotal = tot[3 * k + 1];
+        if (desc[k].total == 0) continue;
+        nmap += (desc[k].total - 1) / 4 + 2 + (desc[k].wtotal - 1) / 4 + 2;
+        longest = std::max(longest, desc[k].total);
+    }
+    int *map = (int *)pdg_pool(ctx, "blocks.maps", std::max<size_t>(1, nmap) * sizeof(int));
+    if (!map) { pdg_set_error("device buffer allocation failed (blocks.maps)"); return PDG_ERR_ALLOC; }
+    for (int k = 0; k < nsub; ++k) {
+        BlockDesc &e = desc[k];
+        if (e.total == 0) continue;
+        e.cbra = map;
+        e.wbra = e.cbra + ((e.total - 1) / 4 + 2);
+        map = e.wbra + ((e.wtotal - 1) / 4 + 2);
+        live.push_back(e);
+        const Sub &u = subs[k];
+        if (ctx->blocks.empty() || ctx->blocks.back().cb != u.cb || ctx->blocks.back().ck != u.ck) {
+            QuartetBlock qb{};
+            qb.cb = u.cb;
+            qb.ck = u.ck;
+            ctx->blocks.push_back(qb);
         }
+        QuartetBlock &qb = ctx->blocks.back();
+        auto &sb = qb.sub[qb.nsub++];
+        sb.total = e.total;
+        sb.wtotal = e.wtotal;
+        sb.offs = e.offs;
+        sb.woffs = e.woffs;
+        sb.cbra = e.cbra;
+        sb.wbra = e.wbra;
+        sb.k0 = e.k0;
+        sb.nk = e.nk;
+        sb.bucket = u.kb;
+        sb.g0 = ctx->bucket_group[u.ck][u.kb];
+        qb.total += sb.total;
+        const int lt = PLA[u.cb] + PLB[u.cb] + PLA[u.ck] + PLB[u.ck];
+        const double per = 20.0 + (lt / 2 + 1) * ncart(PLA[u.cb]) * ncart(PLB[u.cb]) * ncart(PLA[u.ck]) * ncart(PLB[u.ck]);
+        qb.cost += per * ctx->hostNp[u.ck][e.k0] * tot[3 * k + 2];
+    }
+    if (!live.empty()) {
+        Staged up;
+        up.add(live);
+        PDG_CHECK(up.send(ctx, "blocks.desc", &ddesc));
+        const unsigned gx = (unsigned)std::min<long long>(64, ((longest - 1) / 4 + 2 + 255) / 256);
+        { bra_map_kernel<<<dim3(gx, (unsigned)live.size(), 2), 256, 0, ctx->stream>>>((const BlockDesc *)ddesc); pdg_count_launch(); }
+        PDG_CUDA(cudaGetLastError());
     }
     // the launches overlap (ClassFork): the longest go first
     std::stable_sort(ctx->blocks.begin(), ctx->blocks.end(), [](const QuartetBlock &x, const QuartetBlock &y) { return x.cost > y.cost; });

@@ -233,35 +233,6 @@ __device__ __forceinline__ void eri_prim32(const PairRec32 &B, const PairRec32 &
     }
 }
 
-// Contracted raw Cartesian block of one shell quartet.  CUT applies the reference's
-// primitive-quartet cut; the Schwarz diagonal is computed without it, because a primitive pair
-// cut in (ab|ab) can still contribute to (ab|cd) against a compact ket pair.
-template <int LA, int LB, int LC, int LD, bool CUT = true, typename T = double>
-__device__ __forceinline__ void eri_block(const PrimPairs &pp, int pb0, int npb, int pk0, int npk,
-                                          const QuartetGeom &g,
-                                          T (&V)[ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)]) {
-#pragma unroll
-    for (int i = 0; i < ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD); ++i) V[i] = T(0);
-    for (int ib = pb0; ib < pb0 + npb; ++ib) {
-        if constexpr (std::is_same<T, float>::value) {
-            const PairRec32 Bp = load_rec32(pp.rec32, ib);
-            const QuartetGeom32 g32 = geom32(g);
-            for (int ik = pk0; ik < pk0 + npk; ++ik) {
-                const PairRec32 Kp = load_rec32(pp.rec32, ik);
-                if (CUT && Bp.arg + Kp.arg > (float)PDG_PRIMITIVE_CUT) continue;
-                eri_prim32<LA, LB, LC, LD>(Bp, Kp, g32, V);
-            }
-        } else {
-            const double argb = load_arg(pp.rec, ib);
-            const PairRec Bp = load_rec(pp.rec, ib);
-            for (int ik = pk0; ik < pk0 + npk; ++ik) {
-                if (CUT && argb + load_arg(pp.rec, ik) > PDG_PRIMITIVE_CUT) continue;
-                eri_prim<LA, LB, LC, LD, T>(Bp, load_rec(pp.rec, ik), g, V);
-            }
-        }
-    }
-}
-
 __device__ __forceinline__ void load_xyz(const DeviceBasis &bs, int sh, double *r) {
     const int at = bs.sh_atom[sh];
     r[0] = bs.atom_xyz[3 * at];

@@ -80,6 +80,11 @@ extern "C" int pdg_work_estimate(pdg_context *ctx, const char *region, double *f
                                gcx * (m[(size_t)A * ns + C] * m[(size_t)B * ns + D] + m[(size_t)A * ns + D] * m[(size_t)B * ns + C]);
             return ctx->hostQ[cb][ib] * ctx->hostQ[ck][ik] * gam >= ctx->grad_gcut;
         };
+        if (ctx->hostArg.empty() && ctx->npp > 0) {
+            ctx->hostArg.resize(ctx->npp);
+            PDG_CUDA(cudaMemcpyAsync(ctx->hostArg.data(), ctx->pp.arg, ctx->npp * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+            PDG_CUDA(cudaStreamSynchronize(ctx->stream));
+        }
         double w = 0.0;
         long long nq = 0;
         for (const auto &b : ctx->blocks) {
