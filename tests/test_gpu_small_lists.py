@@ -1,0 +1,79 @@
+"""Edges of the size rules: purification sizes, atoms per warp of the one-electron kernels, lanes of short
+quartet lists, and work lists of more bras than one pass of the prefix sums.
+
+Tolerances: integrals, Fock matrices and gradients as in test_gpu_hf.py (1e-10, 1e-8); the purified density
+stops where tr(P - P^2) < 1e-12 before a last squaring step, so that the idempotency error is rounding of
+m-term sums of elements of order one, m^2 eps < 1e-11.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from conftest import ANGSTROM_TO_BOHR
+from pdynamo3_b200 import geometry
+from pdynamo3_b200.basis import ShellTable
+
+pytestmark = pytest.mark.gpu
+
+
+def _context(basis, z, xyz):
+    from pdynamo3_b200.lib import Context
+    ctx = Context(0)
+    ctx.set_basis(ShellTable(basis, z))
+    ctx.set_geometry(xyz)
+    return ctx
+
+
+def _full(packed):
+    n = int((np.sqrt(8 * len(packed) + 1) - 1) / 2)
+    M = np.zeros((n, n))
+    M[np.tril_indices(n)] = packed
+    return M + np.tril(M, -1).T
+
+
+# functions: 4 (one tile), 57 and 72 (either side of one row tile per warp), 126 and 133 (of two), 144 (the
+# largest of the one-launch form) and 152 (GEMMs)
+@pytest.mark.parametrize("basis,waters", [("6-31g_st_cart", 0), ("6-31g_st_cart", 3), ("6-31g_st", 4), ("6-31g_st", 7),
+                                          ("6-31g_st_cart", 7), ("6-31g_st", 8), ("6-31g_st_cart", 8)])
+def test_purified_density_is_a_projector(cuda_device, basis, waters):
+    if waters:
+        z, xyz = geometry.water_cluster(waters, max(3.0, 3.2 * waters ** (1.0 / 3.0)), 7)
+    else:
+        z, xyz = np.array([1, 1]), np.array([[0.0, 0.0, 0.0], [0.0, 0.0, 0.74]])
+    ctx = _context(basis, z, xyz * ANGSTROM_TO_BOHR)
+    P, res = ctx.scf(density_tolerance=1e-9, energy_tolerance=1e-8)
+    S = _full(ctx.one_electron()[0])
+    P = _full(P)
+    assert res.converged
+    assert abs((P * S).sum() - z.sum()) < 1e-9
+    assert np.abs(P @ S @ P - 2.0 * P).max() < 1e-10
+
+
+@pytest.mark.parametrize("natom", [1, 2, 4, 5, 16, 17, 32, 33])
+def test_hydrogen_chains_against_oracle(cuda_device, natom):
+    z = np.ones(natom, dtype=int)
+    rng = np.random.default_rng(natom)
+    xyz = np.stack([1.7 * np.arange(natom), rng.normal(scale=0.3, size=natom), rng.normal(scale=0.3, size=natom)], 1)
+    shells = ShellTable("6-31g_st_cart", z)
+    ctx = _context("6-31g_st_cart", z, xyz)
+    o = oracle.Oracle(shells, xyz)
+    S, H, _ = ctx.one_electron()
+    So, Ho, _ = o.one_electron()
+    assert np.abs(S - So).max() < 1e-10
+    assert np.abs(H - Ho).max() < 1e-9
+    n = len(So)
+    P = 0.2 * rng.normal(size=n)
+    W = 0.2 * rng.normal(size=n)
+    F, _ = ctx.fock_two_electron(P, 1.0)
+    # quartets below a Schwarz bound of 1e-13 are left out: at most norb^2 of them per element, |P| < 1
+    norb = o.n
+    assert np.abs(F - o.fock(P, 1.0)[0]).max() < max(1e-10, 1e-13 * norb ** 2)
+    assert np.abs(ctx.gradients(P, W, 1.0) - o.gradients(P, W)).max() < 1e-8
+
+
+def test_work_list_totals(cuda_device):
+    """12 waters have more than 1024 (ps) pairs: the device's totals against the host's count of the rule."""
+    z, xyz = geometry.water_cluster(12, 7.5, 3)
+    ctx = _context("6-31g_st_cart", z, xyz * ANGSTROM_TO_BOHR)
+    _, res = ctx.scf(maximum_iterations=50)
+    assert res.quartets == ctx.work_estimate("eri_jk")[2]
