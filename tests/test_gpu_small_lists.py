@@ -2,8 +2,9 @@
 quartet lists, and work lists of more bras than one pass of the prefix sums.
 
 Tolerances: integrals, Fock matrices and gradients as in test_gpu_hf.py (1e-10, 1e-8); the purified density
-stops where tr(P - P^2) < 1e-12 before a last squaring step, so that the idempotency error is rounding of
-m-term sums of elements of order one, m^2 eps < 1e-11.
+stops where tr(P - P^2) < 1e-12 before a last squaring step, so that in an orthonormal basis the idempotency error
+is rounding of m-term sums of elements of order one over some 40 steps, below m^2 eps; the tests' limits
+around P S P allow for the condition of S on top.
 """
 import numpy as np
 import pytest
@@ -47,6 +48,30 @@ def test_purified_density_is_a_projector(cuda_device, basis, waters):
     assert res.converged
     assert abs((P * S).sum() - z.sum()) < 1e-9
     assert np.abs(P @ S @ P - 2.0 * P).max() < 1e-10
+
+
+def _stretched_ethene():
+    """C2H4 with bonds 1.6 times the ordinary: a gap of some 0.05 hartree in PBE, 1/400 of the spectrum's width."""
+    c, h = 0.67, 1.09
+    x = [[-c, 0, 0], [c, 0, 0]] + [[s * (c + h * 0.5), t * h * 0.866, 0] for s in (-1, 1) for t in (-1, 1)]
+    return np.array([6, 6, 1, 1, 1, 1]), 1.6 * np.array(x)
+
+
+# iterations of many steps, where rounding errors that a step amplifies would show: molecules of small gaps
+# on either side of the tile counts of the one-launch form
+@pytest.mark.parametrize("basis,molecule", [("6-31g_st_cart", "ethene"), ("6-31g_st", "ethene"), ("6-31g_st_cart", 5),
+                                            ("6-31g_st", 5), ("6-31g_st_cart", 7)])
+def test_purified_density_of_small_gaps(cuda_device, basis, molecule):
+    z, xyz = _stretched_ethene() if molecule == "ethene" else geometry.organic_molecule(molecule, {5: 5, 7: 1}[molecule])
+    ctx = _context(basis, z, xyz * ANGSTROM_TO_BOHR)
+    ctx.set_functional("pbe")
+    ctx.grid_build(3)
+    P, res = ctx.scf(density_tolerance=1e-8, energy_tolerance=1e-7)
+    s, U = np.linalg.eigh(_full(ctx.one_electron()[0]))
+    root = (U * np.sqrt(s)) @ U.T
+    Q = 0.5 * root @ _full(P) @ root  # the lower triangle mirrored: an antisymmetric part shows to first order
+    assert res.converged
+    assert np.abs(Q @ Q - Q).max() < ctx.n ** 2 * np.finfo(float).eps
 
 
 @pytest.mark.parametrize("natom", [1, 2, 4, 5, 16, 17, 32, 33])
