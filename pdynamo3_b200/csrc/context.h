@@ -106,6 +106,9 @@ struct pdg_context {
     double *d_Fout = nullptr;
     int *d_status = nullptr;
 
+    // clusters of the one-launch purification that the device holds, by kernel (purify.cu; -1: not asked yet)
+    int purify_clusters[2] = {-1, -1};
+
     // ---- superposition-of-atomic-densities guess ----
     int guess_sad = 1;
     std::vector<double> occ;               // orbital occupations overriding 2 x nocc (atomic runs only)

@@ -15,7 +15,9 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr int PUR_CTAS = 8, PUR_T = 256;
-constexpr int PUR_MMAX = 144;  // P (row stride 148) and the owned columns of P^2 fill 195 of 227 KB
+// At 128 functions a step takes 12 us here, 18 us as GEMMs; at 129 (three tiles per warp) 22 us against 20 us.
+// P (row stride 132) and the owned rows of P^2 fill 149 KB.
+constexpr int PUR_MMAX = 128;
 
 __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
@@ -167,12 +169,47 @@ __global__ void __cluster_dims__(PUR_CTAS, 1, 1) __launch_bounds__(PUR_T, 1)
 
 }  // namespace
 
-// Whether purify_cluster_kernel takes this size: all that its shared memory holds.  The GEMMs' steps grow
-// slower with the size, but take 11 us at 110 functions.
-bool pdg_purify_fits(int m) { return m <= PUR_MMAX; }
+namespace {
+
+using PurifyKernel = void (*)(int, double *, double *);
+PurifyKernel purify_kernel(int m) { return m <= 64 ? purify_cluster_kernel<1, 1> : purify_cluster_kernel<2, 2>; }
+
+}  // namespace
+
+// How many clusters of the one-launch form for m functions the current device holds at a time; 0 above
+// PUR_MMAX, and where eight such CTAs have no place together (a partitioned device, none at all).
+extern "C" int pdg_purify_clusters(int m) {
+    if (m < 1 || m > PUR_MMAX) return 0;
+    const PurifyKernel kern = purify_kernel(m);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute dims[1];
+    dims[0].id = cudaLaunchAttributeClusterDimension;
+    dims[0].val.clusterDim.x = PUR_CTAS;
+    dims[0].val.clusterDim.y = dims[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(PUR_CTAS);
+    cfg.blockDim = dim3(PUR_T);
+    cfg.dynamicSmemBytes = pur_smem(m);
+    cfg.attrs = dims;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (pdg_allow_max_smem(kern) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+// Whether purify_cluster_kernel takes this size on the context's device (asked once per kernel, for its largest
+// size).
+bool pdg_purify_fits(pdg_context *ctx, int m) {
+    if (m > PUR_MMAX) return false;
+    int &n = ctx->purify_clusters[m <= 64 ? 0 : 1];
+    if (n < 0) n = pdg_purify_clusters(m <= 64 ? 64 : PUR_MMAX);
+    return n > 0;
+}
 
 int pdg_purify_cluster(pdg_context *ctx, int m, double *d_Q, double *d_status) {
-    const auto kern = m <= 64 ? purify_cluster_kernel<1, 1> : m <= 128 ? purify_cluster_kernel<2, 2> : purify_cluster_kernel<3, 3>;
+    const PurifyKernel kern = purify_kernel(m);
     PDG_CUDA(pdg_allow_max_smem(kern));
     { kern<<<PUR_CTAS, PUR_T, pur_smem(m), ctx->stream>>>(m, d_Q, d_status); pdg_count_launch(); }
     PDG_CUDA(cudaGetLastError());

@@ -22,7 +22,7 @@ int pdg_out_to_cart(pdg_context *ctx, const double *Mo, double *Mc);
 int pdg_fock2_scf(pdg_context *ctx, double cx, bool doJ, double *d_F2);
 int pdg_store_packed(pdg_context *ctx, const double *d_full_out, double *packed_host);
 int pdg_gradients_device(pdg_context *ctx, double cx, bool doJ, std::vector<double> &g);
-bool pdg_purify_fits(int m);
+bool pdg_purify_fits(pdg_context *ctx, int m);
 int pdg_purify_cluster(pdg_context *ctx, int m, double *d_Q, double *d_status);
 int pdg_oneint_grad(pdg_context *ctx, const double *d_P, const double *d_W, double *d_grad);
 int pdg_eri_grad(pdg_context *ctx, const double *d_D, double cx, bool doJ, double *d_grad);
@@ -341,7 +341,7 @@ int purify_density(pdg_context *ctx, ScfState &st, const double *F, int nocc, do
     const int grid = (int)std::min<long long>(32, (n + 255) / 256);
     { purify_init_kernel<<<grid, 256, 0, ctx->stream>>>(m, st.T2, rows, nocc, Q); pdg_count_launch(); }
     bool done = false;
-    const bool cluster = pdg_purify_fits(m);
+    const bool cluster = pdg_purify_fits(ctx, m);
     if (cluster) {
         PDG_CHECK(pdg_purify_cluster(ctx, m, Q, sc + 3));
         double t;

@@ -32,8 +32,8 @@ def _full(packed):
     return M + np.tril(M, -1).T
 
 
-# functions: 4 (one tile), 57 and 72 (either side of one row tile per warp), 126 and 133 (of two), 144 (the
-# largest of the one-launch form) and 152 (GEMMs)
+# functions: 4 (one tile), 57 and 72 (either side of one row tile per warp), 126 (below the
+# largest of the one-launch form, 128), 133, 144 and 152 (GEMMs)
 @pytest.mark.parametrize("basis,waters", [("6-31g_st_cart", 0), ("6-31g_st_cart", 3), ("6-31g_st", 4), ("6-31g_st", 7),
                                           ("6-31g_st_cart", 7), ("6-31g_st", 8), ("6-31g_st_cart", 8)])
 def test_purified_density_is_a_projector(cuda_device, basis, waters):
@@ -48,6 +48,11 @@ def test_purified_density_is_a_projector(cuda_device, basis, waters):
     assert res.converged
     assert abs((P * S).sum() - z.sum()) < 1e-9
     assert np.abs(P @ S @ P - 2.0 * P).max() < 1e-10
+
+
+def test_one_launch_form_has_its_cluster(cuda_device):
+    from pdynamo3_b200.lib import load
+    assert [load().pdg_purify_clusters(m) > 0 for m in (1, 64, 65, 128, 129)] == [True, True, True, True, False]
 
 
 def _stretched_ethene():

@@ -2,7 +2,9 @@
 import os
 import re
 
-from conftest import ROOT
+import pytest
+
+from conftest import ROOT, gpu_available
 
 
 def declared_functions():
@@ -29,3 +31,12 @@ def test_version_and_error_string():
     L = lib.load()
     assert L.pdg_version() >= 100
     assert isinstance(L.pdg_last_error(), bytes)
+
+
+@pytest.mark.skipif(gpu_available(), reason="needs a machine without a device")
+def test_purification_without_a_place_for_its_cluster():
+    """Where eight CTAs of the one-launch purification cannot run together (here: no device), the library says
+    so, and an SCF takes the GEMM form, instead of failing in the launch."""
+    from pdynamo3_b200 import lib
+    L = lib.load()
+    assert [L.pdg_purify_clusters(m) for m in (1, 64, 128, 129)] == [0, 0, 0, 0]
