@@ -601,7 +601,8 @@ def run_batch_metric(args):
 
 def tune_eri_lanes(device, rank):
     """The library's tile autotuner (pdg_autotune_eri) run once, untimed, on a mid-size molecule of
-    another seed; its choice of lanes per quartet holds for both timed forms."""
+    another seed; its choice of lanes per quartet, for lists too short for the warp form, holds for both
+    timed forms."""
     from pdynamo3_b200 import workloads
     from pdynamo3_b200.qcmodel import GPUQCEngine
     cands = workloads.batch_molecules(40, seed=BATCH_SEED + 2 + 1000 * rank)
@@ -1094,8 +1095,8 @@ def main():
     ap.add_argument("--rate", type=float, default=4.0, help="stream: arrivals per second")
     ap.add_argument("--rates", default="", help="stream: comma-separated arrival rates to sweep")
     ap.add_argument("--autotune", action="store_true",
-                    help="batch: run the library's ERI lanes autotuner before the timed steps (off: the "
-                         "built-in lanes tables, its choice on a 14-heavy-atom batch molecule)")
+                    help="batch: run the library's ERI lanes autotuner before the timed steps (off: lanes "
+                         "by the length of each list); lists of 8192 items and more have no lanes to tune")
     args = ap.parse_args()
     if args.kernel_case > 0 or args.kernel_molecule >= 0:
         run_kernel_case(args)

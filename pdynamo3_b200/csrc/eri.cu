@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(64) schwarz_kernel(const int n, const int *__r
 struct VariantInit {
     VariantInit() {
         for (int i = 0; i < PDG_NPAIRCLASS; ++i)
-            for (int j = 0; j < PDG_NPAIRCLASS; ++j) pdg_jk_variant[i][j].store(kDefaultLanesV[i][j]);
+            for (int j = 0; j < PDG_NPAIRCLASS; ++j) pdg_jk_variant[i][j].store(-1);
     }
 } g_variant_init;
 
@@ -644,12 +644,12 @@ int pdg_eri_jk_screened(pdg_context *ctx, const double *d_D, double *d_J, double
     return PDG_OK;
 }
 
-// Tile autotuner of the one-thread J+K kernels: for every (bra class, ket class) work list of the
-// current geometry whose kernel splits quartets over lanes, time each candidate lanes-per-bucket
-// table (one warm-up launch, then the best of two CUDA-event-timed launches of a full J+K build of
-// the context's current density into scratch matrices) and keep the fastest in the process-wide
-// table every later build of every context uses.  variants (36 ints, may be NULL) receives the
-// choice per class pair (-1 where nothing was tuned).
+// Tile autotuner of the kernels that split quartets over lanes: for every (bra class, ket class) work list of
+// the current geometry that takes one of their tables (jk_form), time each table (one warm-up launch, then the
+// best of two CUDA-event-timed launches of a full J+K build of the context's current density into scratch
+// matrices) and keep the fastest, which every later list of the class pair below kWarpItems then takes, in
+// every context of the process.  variants (36 ints, may be NULL) receives the choice per class pair (-1
+// where nothing was tuned: no list, a longer list, or a class without tables to choose from).
 extern "C" int pdg_autotune_eri(pdg_context *ctx, int *variants) {
     if (!ctx) { pdg_set_error("pdg_autotune_eri: invalid argument"); return PDG_ERR_ARG; }
     if (ctx->nbf == 0 || !ctx->have_geometry) { pdg_set_error("pdg_autotune_eri: basis and geometry required"); return PDG_ERR_STATE; }
@@ -667,7 +667,7 @@ extern "C" int pdg_autotune_eri(pdg_context *ctx, int *variants) {
     int status = PDG_OK;
     for (const auto &b : ctx->blocks) {
         const int la = PLA[b.cb], lb = PLB[b.cb], lc = PLA[b.ck], ld = PLB[b.ck];
-        if (jk_group(la, lb, lc, ld) > 0 || !jk_split(la, lb, lc, ld)) continue;
+        if (jk_group(la, lb, lc, ld) > 0 || !jk_split(la, lb, lc, ld) || jk_form(b) == kWarpForm) continue;
         JKArgs a;
         a.bra = ctx->pairs[b.cb];
         a.ket = ctx->pairs[b.ck];
@@ -685,7 +685,7 @@ extern "C" int pdg_autotune_eri(pdg_context *ctx, int *variants) {
         a.mixed_cut = ctx->mixed_cut;
         a.count32 = nullptr;
         a.part = 0;
-        int best = kDefaultLanesV[b.cb][b.ck];
+        int best = -1;
         float best_ms = 1e30f;
         for (int v = 0; v < kNLanesV && status == PDG_OK; ++v) {
             a.variant = v;
@@ -712,4 +712,13 @@ extern "C" int pdg_autotune_eri(pdg_context *ctx, int *variants) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     return status;
+}
+
+// What the next J/K build of the current lists launches for a class pair: a table of lanes, kWarpForm, or -1
+// (no list, or the cooperative form).
+extern "C" int pdg_jk_form_of(pdg_context *ctx, int cb, int ck) {
+    if (pdg_ensure_pairs(ctx) != PDG_OK || pdg_build_blocks(ctx, ctx->schwarz_cut) != PDG_OK) return -1;
+    for (const auto &b : ctx->blocks)
+        if (b.cb == cb && b.ck == ck && jk_group(PLA[cb], PLB[cb], PLA[ck], PLB[ck]) == 0) return jk_form(b);
+    return -1;
 }

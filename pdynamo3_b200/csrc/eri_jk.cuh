@@ -35,7 +35,7 @@ struct JKArgs {
     double dcut;         // skip a quartet when Q_AB Q_CD max(relevant dmax) < dcut
     int part;            // 0: every quartet; 1: only bound >= mixed_cut (FP64); 2: only bound < mixed_cut (FP32)
     double mixed_cut;
-    int variant;         // host side: lanes-per-bucket table of the launch (-1: the tuned table)
+    int variant;         // host side: lanes-per-bucket table of the launch (-1: by jk_form)
     unsigned long long *count32;  // optional: running count of quartets evaluated in FP32
 };
 
@@ -71,11 +71,11 @@ __host__ __device__ constexpr int jk_group(int la, int lb, int lc, int ld) {
 __host__ __device__ constexpr bool jk_split(int la, int lb, int lc, int ld) {
     return ncart(la) * ncart(lb) * ncart(lc) * ncart(ld) <= 36;
 }
-// Lanes per quartet by ket bucket for the small-block classes: five candidate tables, one chosen per
-// (bra class, ket class) by pdg_autotune_eri.  The default per class pair (pair classes ss, ps, pp,
-// ds, dp, dd) is the autotuner's choice on a 14-heavy-atom organic molecule in B3LYP/6-31G*
-// (Cartesian): table 3 (2-16 lanes) for (ss|ss), table 0 for (dp|ss) and (dd|ss), table 1 for the
-// rest.
+// Lanes per quartet by ket bucket for the small-block classes in lists below kWarpItems: five tables, taken
+// by the length of the list (jk_form) from the class pair's first one on (pair classes ss, ps, pp, ds, dp,
+// dd), or as pdg_autotune_eri chose.  The first ones are what it chose on a 14-heavy-atom organic molecule in
+// B3LYP/6-31G* (Cartesian) when its lists took tables: table 3 (2-16 lanes) for (ss|ss), table 0 for (dp|ss)
+// and (dd|ss), table 1 for the rest.
 constexpr int kNLanesV = 5;
 constexpr int kSplitLanesV[kNLanesV][PDG_NBUCKET] = {
     {1, 1, 1, 2, 2}, {1, 1, 2, 4, 4}, {1, 2, 4, 8, 8}, {2, 4, 8, 16, 16}, {4, 8, 16, 32, 32}};
@@ -97,10 +97,28 @@ constexpr int kWideLanes[kNWide][PDG_NBUCKET] = {{1, 1, 1, 1, 1}, {1, 2, 2, 2, 2
 
 }  // namespace
 
-// The table of each (bra class, ket class) in use by every context of the process.
+// The table that pdg_autotune_eri chose for each (bra class, ket class), for every context of the process (-1:
+// none, by the length of the list).
 extern std::atomic<int> pdg_jk_variant[PDG_NPAIRCLASS][PDG_NPAIRCLASS];
 
 namespace {
+
+// The form of a list of a class pair without cooperative kernel: kWarpForm, or the table of lanes (of
+// kSplitLanesV or kWideLanes).
+constexpr int kWarpForm = 8;
+inline int jk_form(const QuartetBlock &b) {
+    if (pdg_warp_items(b) >= kWarpItems) return kWarpForm;
+    int v = 0;
+    if (jk_split(PLA[b.cb], PLB[b.cb], PLA[b.ck], PLB[b.ck])) {
+        v = pdg_jk_variant[b.cb][b.ck].load(std::memory_order_relaxed);
+        if (v >= 0) return v;
+        v = kDefaultLanesV[b.cb][b.ck];
+        while (v + 1 < kNLanesV && pdg_work_threads(b, kSplitLanesV[v + 1]) <= kLaneThreads) ++v;
+    } else {
+        while (v + 1 < kNWide && pdg_work_threads(b, kWideLanes[v + 1]) <= kLaneThreads / 2) ++v;
+    }
+    return v;
+}
 
 constexpr double TWO_PI_POW_2P5 = 34.986836655249725;  // 2 pi^(5/2)
 
@@ -913,26 +931,15 @@ void launch_jk_p(JKArgs a, const QuartetBlock &b, bool doJ, bool doK, cudaStream
         else if (doJ) launch_jk_group<LA, LB, LC, LD, G, true, false, T>(a, b, st);
         else launch_jk_group<LA, LB, LC, LD, G, false, true, T>(a, b, st);
     } else {
-        if (a.variant < 0 && pdg_warp_items(b) >= kWarpItems) {
+        const int v = a.variant >= 0 ? a.variant : jk_form(b);
+        if (v == kWarpForm) {
             const long long blocks = pdg_fill_warp_work(a.work, b);
             if (doJ && doK) { eri_jk_warp_kernel<LA, LB, LC, LD, true, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
             else if (doJ) { eri_jk_warp_kernel<LA, LB, LC, LD, true, false, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
             else { eri_jk_warp_kernel<LA, LB, LC, LD, false, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
             return;
         }
-        long long blocks;
-        if constexpr (jk_split(LA, LB, LC, LD)) {
-            int v = a.variant;
-            if (v < 0) {
-                v = pdg_jk_variant[CB][CK].load(std::memory_order_relaxed);
-                while (v + 1 < kNLanesV && pdg_work_threads(b, kSplitLanesV[v + 1]) <= kLaneThreads) ++v;
-            }
-            blocks = pdg_fill_work(a.work, b, kSplitLanesV[v]);
-        } else {
-            int v = 0;
-            while (v + 1 < kNWide && pdg_work_threads(b, kWideLanes[v + 1]) <= kLaneThreads / 2) ++v;
-            blocks = pdg_fill_work(a.work, b, kWideLanes[v]);
-        }
+        const long long blocks = pdg_fill_work(a.work, b, jk_split(LA, LB, LC, LD) ? kSplitLanesV[v] : kWideLanes[v]);
         if (doJ && doK) { eri_jk_kernel<LA, LB, LC, LD, true, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
         else if (doJ) { eri_jk_kernel<LA, LB, LC, LD, true, false, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }
         else { eri_jk_kernel<LA, LB, LC, LD, false, true, T><<<(unsigned)blocks, 128, 0, st>>>(a); pdg_count_launch(); }

@@ -110,3 +110,16 @@ def test_work_list_totals(cuda_device):
     ctx = _context("6-31g_st_cart", z, xyz * ANGSTROM_TO_BOHR)
     _, res = ctx.scf(maximum_iterations=50)
     assert res.quartets == ctx.work_estimate("eri_jk")[2]
+
+
+def test_builds_launch_what_the_autotuner_reports(cuda_device):
+    """4 waters have short lists only; 8 waters long ones too, which have no lanes to tune."""
+    for waters, long_lists in ((4, False), (8, True)):
+        z, xyz = geometry.water_cluster(waters, max(3.0, 3.2 * waters ** (1.0 / 3.0)), 3)
+        ctx = _context("6-31g_st_cart", z, xyz * ANGSTROM_TO_BOHR)
+        ctx.fock_two_electron(np.full(ctx.npacked(), 0.01), 1.0)
+        tuned = ctx.autotune_eri()
+        forms = {(b, k): ctx.L.pdg_jk_form_of(ctx.h, b, k) for b in range(6) for k in range(b + 1)}
+        assert tuned and all(forms[p] == v for p, v in tuned.items())
+        assert ((0, 0) not in tuned) == long_lists == (forms[0, 0] == 8)
+        ctx.close()
