@@ -38,6 +38,7 @@ void *pdg_pool(pdg_context *ctx, const char *name, size_t bytes) {
     const size_t want = bytes + bytes / 8 + 256;  // headroom so small growth does not reallocate
     if (cudaMalloc(&e.first, want) != cudaSuccess) {
         e.first = nullptr;
+        cudaGetLastError();  // the caller reports it; the next call's check of its launches must not
         return nullptr;
     }
     e.second = want;

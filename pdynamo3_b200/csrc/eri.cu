@@ -184,8 +184,7 @@ __global__ void __launch_bounds__(128) pair_fill_kernel(int n, const int *__rest
 // the primitive pairs of each shell pair and sorts; the device forms them and the bounds, between two
 // transfers up and one down (formed on the host and sent array by array, each waited for: 8 ms of a new
 // geometry of 32 waters, 1.6 ms of one of 4).
-int pdg_ensure_pairs(pdg_context *ctx) {
-    if (ctx->pairs[0].shA || ctx->pp.a) return PDG_OK;
+static int build_pairs(pdg_context *ctx) {
     ProfScope prof(ctx, "pairs");
     const auto &sh = ctx->shells;
     const int ns = (int)sh.size();
@@ -341,6 +340,14 @@ int pdg_ensure_pairs(pdg_context *ctx) {
         pl.goff = dg;
     }
     return PDG_OK;
+}
+
+// A failure part of the way (device memory) leaves no half of the lists: the next call starts over.
+int pdg_ensure_pairs(pdg_context *ctx) {
+    if (ctx->pp.a) return PDG_OK;
+    const int status = build_pairs(ctx);
+    if (status != PDG_OK) pdg_free_pairs(ctx);
+    return status;
 }
 
 // One (bra class, ket class, ket bucket) of the work list while it is built.
@@ -717,6 +724,7 @@ extern "C" int pdg_autotune_eri(pdg_context *ctx, int *variants) {
 // What the next J/K build of the current lists launches for a class pair: a table of lanes, kWarpForm, or -1
 // (no list, or the cooperative form).
 extern "C" int pdg_jk_form_of(pdg_context *ctx, int cb, int ck) {
+    if (!ctx || ctx->nbf == 0 || !ctx->have_geometry) return -1;
     if (pdg_ensure_pairs(ctx) != PDG_OK || pdg_build_blocks(ctx, ctx->schwarz_cut) != PDG_OK) return -1;
     for (const auto &b : ctx->blocks)
         if (b.cb == cb && b.ck == ck && jk_group(PLA[cb], PLB[cb], PLA[ck], PLB[ck]) == 0) return jk_form(b);

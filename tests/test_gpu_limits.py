@@ -4,6 +4,8 @@ the documented status before any device work, and the context stays usable.
 * a shell above d (f functions): PDG_ERR_UNSUPPORTED from pdg_basis_upload;
 * a DFT grid for more than 256 atoms: PDG_ERR_UNSUPPORTED from pdg_grid_build;
 * out-of-order calls (a Fock build without a geometry): PDG_ERR_STATE;
+* device memory that runs out while the pair lists of a geometry are built: PDG_ERR_ALLOC (or the runtime's
+  error), and the same call works once there is memory again;
 * empty point sets for the functional entry points: no work, empty results;
 * an unknown functional name: PDG_ERR_UNSUPPORTED.
 """
@@ -81,3 +83,44 @@ def test_out_of_order_calls_and_unknown_names_are_refused(cuda_device):
     for fn in (xc_evaluate, xc_evaluate_static):
         f, vr, vs = fn("pbe", np.zeros(0), np.zeros(0))
         assert f.size == vr.size == vs.size == 0
+
+
+def test_pair_lists_start_over_after_a_failed_allocation(cuda_device):
+    """0 to 24 MB are left of the device's memory, where the lists of 24 waters take some 12 MB in a dozen
+    allocations, so that now this one fails, now that; the call afterwards, with memory, gives what a fresh
+    context gives."""
+    import torch
+    from pdynamo3_b200 import geometry
+    from pdynamo3_b200.lib import PDG_ERR_ALLOC, PDG_ERR_CUDA, Context, PDGError
+    z, xyz = geometry.water_cluster(24, 3.2 * 24 ** (1.0 / 3.0), 5)
+    shells = ShellTable("6-31g_st_cart", z)
+
+    def context():
+        ctx = Context(0)
+        ctx.set_basis(shells)
+        ctx.set_geometry(xyz * ANGSTROM_TO_BOHR)
+        return ctx
+
+    ref = context()
+    P = 0.01 * np.random.default_rng(1).normal(size=ref.npacked())
+    S0, H0, _ = ref.one_electron()
+    F0, _ = ref.fock_two_electron(P, 1.0)
+    ref.close()
+    refused = 0
+    for left in range(0, 26, 2):
+        ctx = context()
+        free = torch.cuda.mem_get_info()[0]
+        filler = torch.empty(max(0, free - left * 2 ** 20), dtype=torch.uint8, device="cuda")
+        try:
+            ctx.fock_two_electron(P, 1.0)
+        except PDGError as err:
+            assert err.status in (PDG_ERR_ALLOC, PDG_ERR_CUDA)
+            refused += 1
+        finally:
+            del filler
+            torch.cuda.empty_cache()
+        S, H, _ = ctx.one_electron()
+        F, _ = ctx.fock_two_electron(P, 1.0)
+        assert np.array_equal(S, S0) and np.abs(H - H0).max() < 1e-10 and np.abs(F - F0).max() < 1e-10
+        ctx.close()
+    assert refused > 0
