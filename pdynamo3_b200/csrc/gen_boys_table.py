@@ -4,9 +4,10 @@ F_m(x) = integral_0^1 t^(2m) exp(-x t^2) dt, m = 0 .. MMAX, on [0, XMAX): interv
 the polynomial in t in [-1, 1] (t = 2 (x - x_mid) / H) through the Chebyshev nodes, monomial
 coefficients c_0 .. c_(N-1) contiguous, so that one evaluation reads one aligned run of N values.
 FP64: H = 1/8, 8 coefficients (one 64-byte run).  The interpolation error is below
-2 (H/4)^8 / 8! max|F_m^(8)| = 4.5e-17 / (2 m + 17), i.e. below 1e-17 of F_m(0) = 1 / (2 m + 1); for
-larger x the derivatives fall faster than F_m.  FP32: H = 1/8, 4 coefficients (one 16-byte run), error
-below 2 (H/4)^4 / 4! / (2 m + 9) = 8e-8 / (2 m + 9), below half a unit in the last place of F_m(0).
+2 (H/4)^8 / 8! max|F_m^(8)| = 4.5e-17 / (2 m + 17), i.e. below 2e-17 of F_m(0) = 1 / (2 m + 1) for m <= 5;
+for larger x the derivatives fall faster than F_m.  FP32: H = 1/8, 4 coefficients (one 16-byte run), error
+below 2 (H/4)^4 / 4! / (2 m + 9) = 8e-8 / (2 m + 9), below one unit in the last place of F_m(0), and below
+half a unit for m <= 3.
 From XMAX on, exp(-x) is below 3e-22 and F_m is Gamma(m + 1/2) / (2 x^(m + 1/2)) to double precision.
 
 Values are taken at 40 digits with mpmath (incomplete gamma function).  Re-run:  python gen_boys_table.py

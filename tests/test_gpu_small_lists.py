@@ -1,5 +1,6 @@
 """Edges of the size rules: purification sizes, atoms per warp of the one-electron kernels, lanes of short
-quartet lists, and work lists of more bras than one pass of the prefix sums.
+quartet lists, the line between short and long lists, and work lists of more bras than one pass of the prefix
+sums.
 
 Tolerances: integrals, Fock matrices and gradients as in test_gpu_hf.py (1e-10, 1e-8); the purified density
 stops where tr(P - P^2) < 1e-12 before a last squaring step, so that in an orthonormal basis the idempotency error
@@ -123,3 +124,46 @@ def test_builds_launch_what_the_autotuner_reports(cuda_device):
         assert tuned and all(forms[p] == v for p, v in tuned.items())
         assert ((0, 0) not in tuned) == long_lists == (forms[0, 0] == 8)
         ctx.close()
+
+
+@pytest.fixture(scope="module")
+def four_atoms():
+    """s, p and d shells on four atoms: geometry, densities and the oracle's Fock matrices and gradients."""
+    from test_gpu_limits import RawShells
+    xyz = np.array([[0.0, 0.1, 0.0], [1.9, 0.2, 0.1], [-0.3, 1.7, 0.4], [0.4, -0.2, 2.1]])
+    o = oracle.Oracle(RawShells([3, 1, 2, 1], _spd_shells(4)), xyz)
+    rng = np.random.default_rng(17)
+    npk = o.n * (o.n + 1) // 2
+    P, W = 0.3 * rng.normal(size=npk), 0.1 * rng.normal(size=npk)
+    kinds = ((1.0, True), (0.0, True), (1.0, False))  # J and K, J, K
+    return xyz, P, W, {k: (o.fock(P, *k)[0], o.gradients(P, W, *k)) for k in kinds}
+
+
+def _spd_shells(n):
+    return [s for a in range(n) for s in ((a, 0, 0, [9.0, 1.9, 0.5], [0.1, 0.4, 0.6]), (a, 0, 0, [0.17], [1.0]),
+                                          (a, 1, 1, [2.1, 0.4], [0.4, 0.7]), (a, 2, 2, [0.8], [1.0]))]
+
+
+# The quartets of the four atoms alone (short lists, lanes split over primitives) and among 36 centres without
+# charge, density or weight (long lists of every class, one quartet per lane): their Fock block and
+# gradient are the same.  In the mixed mode with every quartet in FP32 an element is a sum of some 44^2
+# products of 0.3 and an integral of order one, each with a few roundings of 6e-8: 1e-4.
+@pytest.mark.parametrize("ghosts,mixed_cut,ftol,gtol", [(0, 0.0, 1e-10, 1e-8), (36, 0.0, 1e-10, 1e-8),
+                                                        (0, 1e9, 1e-4, 1e-4), (36, 1e9, 1e-4, 1e-4)])
+def test_short_and_long_lists_against_oracle(cuda_device, four_atoms, ghosts, mixed_cut, ftol, gtol):
+    from test_gpu_limits import RawShells
+    from pdynamo3_b200.lib import Context
+    xyz, P, W, expected = four_atoms
+    ctx = Context(0)
+    ctx.set_basis(RawShells([3, 1, 2, 1] + [0] * ghosts, _spd_shells(4 + ghosts)))
+    ctx.set_geometry(np.concatenate([xyz, np.random.default_rng(5).uniform(-4.0, 4.0, size=(ghosts, 3))]))
+    ctx.set_eri_options(precision_mode=1 if mixed_cut else 0, mixed_cut=mixed_cut or 1e-6)
+    pad = lambda v: np.concatenate([v, np.zeros(ctx.npacked() - len(v))])  # noqa: E731
+    for (cx, coulomb), (Fo, go) in expected.items():
+        F, _ = ctx.fock_two_electron(pad(P), cx, coulomb)
+        assert np.abs(F[:len(P)] - Fo).max() < ftol
+        g = ctx.gradients(pad(P), pad(W), cx, coulomb)
+        assert np.abs(g[:4] - go).max() < gtol
+        assert np.abs(g[4:]).max(initial=0.0) < 1e-12
+    forms = {ctx.L.pdg_jk_form_of(ctx.h, b, k) for b in range(6) for k in range(b + 1)} - {-1}
+    assert forms == {8} if ghosts else 8 not in forms
