@@ -319,7 +319,7 @@ struct RhoArgs {
     const long long *foff, *voff;
     const int *fun;
     const double *pts, *bval, *D;  // D: scaled Cartesian density D' (n x n)
-    int n, kind, chunk;
+    int n, kind;
     double rho_tol;
     double *pcoef, *pF, *red;  // red[0] += E_xc, red[1] += integrated rho
     int *skip;
@@ -680,7 +680,7 @@ struct GradArgs {
     const double *Z;  // Zg rows of each block at foff[b] * BLK
     const int *skip;
     DeviceBasis bs;
-    int n, chunk;
+    int n;
     double *grad;
 };
 
@@ -1400,22 +1400,7 @@ static double shell_radius(const pdg_context *ctx, const HostShell &h, double to
     return hi;
 }
 
-extern "C" int pdg_grid_build(pdg_context *ctx, int accuracy, int n_radial, int angular_l, long long *n_points) {
-    if (!ctx || accuracy < 1 || accuracy > 5 || n_radial < 0 || angular_l < 0) {
-        pdg_set_error("pdg_grid_build: invalid argument");
-        return PDG_ERR_ARG;
-    }
-    if (ctx->nbf == 0 || !ctx->have_geometry) { pdg_set_error("pdg_grid_build: basis and geometry required"); return PDG_ERR_STATE; }
-    if (ctx->natom > 256) { pdg_set_error("pdg_grid_build: more than 256 atoms"); return PDG_ERR_UNSUPPORTED; }
-    cudaSetDevice(ctx->device);
-    ProfScope prof(ctx, "grid_build");
-    if (!ctx->xc) ctx->xc = new XCData();
-    ctx->xc->accuracy = accuracy;
-    ctx->xc->nr = n_radial;
-    ctx->xc->lq = angular_l;
-    delete ctx->grid;
-    ctx->grid = new GridData();
-    GridData &G = *ctx->grid;
+static int fill_grid(pdg_context *ctx, GridData &G, int accuracy, int n_radial, int angular_l, long long *n_points) {
     const int acc = accuracy - 1;
     G.bf_tol = kBfTol[acc];
     G.rho_tol = kRhoTol[acc];
@@ -1596,6 +1581,26 @@ extern "C" int pdg_grid_build(pdg_context *ctx, int accuracy, int n_radial, int 
     return PDG_OK;
 }
 
+extern "C" int pdg_grid_build(pdg_context *ctx, int accuracy, int n_radial, int angular_l, long long *n_points) {
+    if (!ctx || accuracy < 1 || accuracy > 5 || n_radial < 0 || angular_l < 0) {
+        pdg_set_error("pdg_grid_build: invalid argument");
+        return PDG_ERR_ARG;
+    }
+    if (ctx->nbf == 0 || !ctx->have_geometry) { pdg_set_error("pdg_grid_build: basis and geometry required"); return PDG_ERR_STATE; }
+    if (ctx->natom > 256) { pdg_set_error("pdg_grid_build: more than 256 atoms"); return PDG_ERR_UNSUPPORTED; }
+    cudaSetDevice(ctx->device);
+    ProfScope prof(ctx, "grid_build");
+    if (!ctx->xc) ctx->xc = new XCData();
+    ctx->xc->accuracy = accuracy;
+    ctx->xc->nr = n_radial;
+    ctx->xc->lq = angular_l;
+    delete ctx->grid;
+    ctx->grid = new GridData();
+    const int status = fill_grid(ctx, *ctx->grid, accuracy, n_radial, angular_l, n_points);
+    if (status != PDG_OK) pdg_free_dft(ctx);  // (device memory) no half of a grid: the next quadrature builds it again
+    return status;
+}
+
 // Algorithmic FLOPs and resident-value bytes of one call of the XC density or V_xc kernel.
 double pdg_grid_work(const pdg_context *ctx, const char *region, double *bytes) {
     *bytes = 0.0;
@@ -1617,8 +1622,6 @@ static int ensure_grid(pdg_context *ctx) {
     return pdg_grid_build(ctx, ctx->xc ? ctx->xc->accuracy : 3, ctx->xc ? ctx->xc->nr : 0, ctx->xc ? ctx->xc->lq : 0, &n);
 }
 
-static int chunk_for(int nf) { return nf * 16 * 8 <= 200 * 1024 ? 16 : 8; }
-
 // Quadrature Fock: adds N V_xc N into the normalised Cartesian matrix d_F from the scaled density
 // in ctx->d_D; returns E_xc and the integrated density.
 int pdg_dft_fock_device(pdg_context *ctx, double *d_F, double *exc, double *rho) {
@@ -1631,7 +1634,7 @@ int pdg_dft_fock_device(pdg_context *ctx, double *d_F, double *exc, double *rho)
     if (G.nblk > 0) {
         RhoArgs a;
         a.nblk = G.nblk; a.bstart = G.bstart; a.bcount = G.bcount; a.foff = G.foff; a.voff = G.voff; a.fun = G.fun;
-        a.pts = G.pts; a.bval = G.bval; a.D = ctx->d_D; a.n = n; a.kind = X.kind; a.chunk = chunk_for(G.max_nf);
+        a.pts = G.pts; a.bval = G.bval; a.D = ctx->d_D; a.n = n; a.kind = X.kind;
         a.rho_tol = G.rho_tol; a.pcoef = X.pcoef; a.pF = X.pF; a.red = X.red; a.skip = G.skip;
         {
             ProfScope prof(ctx, "xc_rho");
@@ -1679,7 +1682,7 @@ int pdg_dft_grad_device(pdg_context *ctx, double *d_grad) {
     GradArgs a;
     a.bstart = G.bstart; a.bcount = G.bcount; a.batom = G.batom; a.foff = G.foff; a.voff = G.voff; a.fun = G.fun;
     a.pts = G.pts; a.bval = G.bval; a.pcoef = X.pcoef; a.D = ctx->d_D; a.skip = G.skip; a.bs = ctx->dbasis;
-    a.n = ctx->nbf; a.chunk = 0; a.grad = d_grad;
+    a.n = ctx->nbf; a.grad = d_grad;
     VxcArgs v;  // Zg = c . grad B rows for the W product
     v.bcount = G.bcount; v.bstart = G.bstart; v.foff = G.foff; v.voff = G.voff; v.fun = G.fun; v.bval = G.bval;
     v.pcoef = X.pcoef; v.skip = G.skip; v.n = ctx->nbf; v.V = nullptr; v.c0scale = 0.0;

@@ -6,6 +6,7 @@ the documented status before any device work, and the context stays usable.
 * out-of-order calls (a Fock build without a geometry): PDG_ERR_STATE;
 * device memory that runs out while the pair lists of a geometry are built: PDG_ERR_ALLOC (or the runtime's
   error), and the same call works once there is memory again;
+* the same for the grid: PDG_ERR_ALLOC, and the next quadrature builds it;
 * empty point sets for the functional entry points: no work, empty results;
 * an unknown functional name: PDG_ERR_UNSUPPORTED.
 """
@@ -122,5 +123,43 @@ def test_pair_lists_start_over_after_a_failed_allocation(cuda_device):
         S, H, _ = ctx.one_electron()
         F, _ = ctx.fock_two_electron(P, 1.0)
         assert np.array_equal(S, S0) and np.abs(H - H0).max() < 1e-10 and np.abs(F - F0).max() < 1e-10
+        ctx.close()
+    assert refused > 0
+
+
+def test_grid_starts_over_after_a_failed_allocation(cuda_device):
+    """8 MB to 512 MB are left for the grid of 4 waters, which takes some 400 MB in all."""
+    import torch
+    from pdynamo3_b200 import geometry
+    from pdynamo3_b200.lib import PDG_ERR_ALLOC, PDG_ERR_CUDA, Context, PDGError
+    z, xyz = geometry.water_cluster(4, 5.1, 0)
+
+    def context():
+        ctx = Context(0)
+        ctx.set_basis(ShellTable("6-31g_st_cart", z))
+        ctx.set_geometry(xyz * ANGSTROM_TO_BOHR)
+        ctx.set_functional("pbe")
+        return ctx
+
+    ref = context()
+    ref.grid_build(3)
+    P = np.zeros(ref.npacked())
+    P[[i * (i + 3) // 2 for i in range(ref.n)]] = 0.5
+    F0, exc0, n0 = ref.fock_quadrature(P)
+    ref.close()
+    refused = 0
+    for left in (8, 32, 64, 128, 256, 512):
+        ctx = context()
+        filler = torch.empty(max(0, torch.cuda.mem_get_info()[0] - left * 2 ** 20), dtype=torch.uint8, device="cuda")
+        try:
+            ctx.grid_build(3)
+        except PDGError as err:
+            assert err.status in (PDG_ERR_ALLOC, PDG_ERR_CUDA)
+            refused += 1
+        finally:
+            del filler
+            torch.cuda.empty_cache()
+        F, exc, n = ctx.fock_quadrature(P)
+        assert np.abs(F - F0).max() < 1e-10 and abs(exc - exc0) < 1e-9 and abs(n - n0) < 1e-9
         ctx.close()
     assert refused > 0
