@@ -165,11 +165,15 @@ struct ProfScope {
 // Launches of independent class kernels (all of which only add to their outputs) on the context's stream
 // and the streams beside it, so that one class's blocks fill the SMs that another's last blocks leave
 // idle: a two-electron build is 21 launches in a row, and those of a small molecule hold a few blocks that
-// wait on their longest quartet (J/K of 4 waters 1.22 -> 0.41 ms, of 42 atoms in B3LYP 13.3 -> 11.4 ms; HF
-// gradient of 2 waters 2.55 -> 1.27 ms; HF energy of one water 21.5 -> 13.1 ms).  stream() gives the stream with the least work so far, ordered after
-// what the context's stream holds at that point; the destructor orders the context's stream after all
-// of them, on error paths too.  Without the side streams (their creation failed) everything goes to the
-// context's stream.
+// wait on their longest quartet.  On one stream and on these eight, the same kernels: J/K of 4 waters 0.65 and
+// 0.23 ms, of 42 atoms (B3LYP) 13.0 and 11.1 ms; HF gradient of 2 waters 0.88 and 0.29 ms; first SCF of a
+// context with one water 9.2 and 6.1 ms, although its context and those of the guess's atoms each make the
+// streams first (0.3 ms).  With eight molecules served at a time the chip is full either way: 1.45 and 1.30
+// against 1.27 and 1.35 molecules/s in two runs of 64 each, a difference within the runs' spread; with one at
+// a time 1.62 against 1.44.
+// stream() gives the stream with the least work so far, ordered after what the context's stream holds at that
+// point; the destructor orders the context's stream after all of them, on error paths too.  Without the side
+// streams (their creation failed) everything goes to the context's stream.
 struct ClassFork {
     pdg_context *c;
     bool forked[pdg_context::kSideStreams]{};

@@ -629,14 +629,18 @@ constexpr int PLB[PDG_NPAIRCLASS] = {0, 0, 1, 0, 1, 2};
 
 // Lanes per quartet of the one-thread gradient form by ket bucket: the buckets with many primitive
 // pairs split their primitive quartets.  A list of few quartets takes the rows of more lanes while its
-// threads stay below kGradLaneThreads, about those that fit the chip at the kernels' registers: the launch
-// then lasts as long as its longest quartet, 0.6 ms for (pp|pp) at two lanes.
+// threads stay below kGradLaneThreads, about those that fit the chip's 148 SMs at the kernels' registers: the
+// launch then lasts as long as its longest quartet, 0.6 ms for (pp|pp) at two lanes.  Gradients with the first
+// row alone, with this limit and with eight times it: one water 275, 118, 118 us; 4 waters 824, 483, 544; 8
+// waters 3040, 1809, 2006; a molecule of 8 heavy atoms 6.14, 5.14, 5.22 ms.
 constexpr int kNGradLanes = 4;
 constexpr int kGradLanes[kNGradLanes][PDG_NBUCKET] = {{1, 1, 2, 4, 4}, {1, 2, 4, 8, 8}, {2, 4, 8, 16, 16}, {4, 8, 16, 32, 32}};
 constexpr long long kGradLaneThreads = 148 * 256;
 // Lists of at least this many (bra, ket group) items take the warp-per-bra form: every SM then has its
 // resident warps (8 to 16 at these register counts) more than once over; below it one lane per quartet
-// would leave SMs idle.
+// would leave SMs idle.  Gradients with the line at 1024, 4096, 16384 items and with no warp form at all: 4 waters
+// 584, 472, 468, 469 us; 8 waters 2.84, 2.01, 2.11, 2.17 ms; 12 waters 4.22, 3.64, 3.64, 3.79; 42 atoms 29.2, 29.1,
+// 28.8, 31.3 (the mixed mode alike).
 constexpr long long kGradWarpItems = 4096;
 
 template <int CB, int CK>

@@ -84,13 +84,17 @@ constexpr int kDefaultLanesV[PDG_NPAIRCLASS][PDG_NPAIRCLASS] = {
     {1, 1, 1, 1, 1, 1}, {0, 1, 1, 1, 1, 1}, {0, 1, 1, 1, 1, 1}};
 // Lists of at least this many (bra, ket group) items take the warp-per-bra form; one lane then walks all
 // primitives of a quartet, so a shorter list leaves the chip waiting for its longest quartets and keeps
-// several lanes per quartet (4 waters: 1.20 ms so, 1.36 ms with the line at 2368 items).
+// several lanes per quartet.  J+K builds with the line at 2368, 8192, 32768 items and with no warp form at
+// all: 4 waters 349, 231, 233, 233 us; 6 waters 626, 631, 493, 490; 8 waters 808, 854, 936, 936; 16 waters 4096,
+// 4144, 4375, 5338; 42 atoms 11.13, 11.12, 11.47, 14.41 ms (the mixed mode alike).
 constexpr long long kWarpItems = 8192;
 // A list of few quartets takes the tables of more lanes while its threads stay below kLaneThreads, one to
-// two times those that fit the chip at the kernels' registers: the launch then lasts as long as its longest
-// quartet, and one lane takes 0.2 ms for the 81 primitive quartets of a (pp|pp) one.  Lanes beyond that
+// two times those that fit the chip's 148 SMs at the kernels' registers: the launch then lasts as long as its
+// longest quartet, and one lane takes 0.2 ms for the 81 primitive quartets of a (pp|pp) one.  Lanes beyond that
 // only repeat the quartets' preambles.  The same for the classes of wide blocks, from one lane per
-// quartet and at half the threads (255 registers).
+// quartet and at half the threads (255 registers).  J+K builds with no more lanes than the first table's, with
+// this limit and with eight times it: one water 315, 162, 159 us; 4 waters 341, 234, 242; 8 waters 917, 860, 1091;
+// 16 heavy and hydrogen atoms (5 heavy) 544, 525, 630.
 constexpr long long kLaneThreads = 148 * 1024;
 constexpr int kNWide = 4;
 constexpr int kWideLanes[kNWide][PDG_NBUCKET] = {{1, 1, 1, 1, 1}, {1, 2, 2, 2, 2}, {2, 4, 4, 4, 4}, {4, 8, 8, 8, 8}};

@@ -2,11 +2,10 @@
 //
 // Replaces GaussianBasisContainerIntegrals_f1KOf1i / _f1KOf1R1
 // (GaussianBases/__extensions__/csource/GaussianBasisContainerIntegrals_f1Xg1.c:233,298) and
-// _f2Cm1V / _f2Cm1R1 (GaussianBasisContainerIntegrals_f2Cp1.c:104,30).  One thread per shell
-// pair; overlap and kinetic by the Obara-Saika recursion, electron-nuclear attraction by
-// Rys quadrature with the nucleus as a narrow Gaussian charge, as the reference models it.
-// Raw Cartesian integrals; the
-// per-component normalisation is applied by the caller (N S N).
+// _f2Cm1V / _f2Cm1R1 (GaussianBasisContainerIntegrals_f2Cp1.c:104,30).  One warp per shell
+// pair; overlap and kinetic by the Obara-Saika recursion, electron-nuclear attraction by Boys
+// functions and Hermite sums with the nucleus as a narrow Gaussian charge, as the reference models it.
+// Raw Cartesian integrals; the per-component normalisation is applied by the caller (N S N).
 #include "context.h"
 #include "md.cuh"
 
